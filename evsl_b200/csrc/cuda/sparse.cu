@@ -1102,10 +1102,13 @@ int evslcu::chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, d
 //   0  SELL-32, loop form            1  SELL-32, unrolled
 //   2  pattern table (global), unrolled   3  pattern table (global), loop form
 //   4  pattern table (constant), loop form  5  pattern table (constant), unrolled
+//   6  the merged stencil (stencil.cu) or, for a dictionary that does not merge
+//      into one, the constant table through per-row descriptors
 // Which is fastest depends on the size of the matrix (latency-bound small
 // operators favour the unrolled forms, L2-bound large ones the constant
 // table), so the first filter call on a matrix times every allowed variant on
-// scratch vectors and keeps the fastest.
+// scratch vectors and keeps the fastest.  A matrix with a merged stencil needs
+// no timing: that form was the fastest at every size measured (stencil.cu).
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -1123,7 +1126,7 @@ bool cheb_variant_ok(const evslcu_mat *A, int v) {
     case 3: return pat;
     case 4: return pconst;
     case 5: return pconst && unroll_width(A->pat_maxlen) > 0;
-    case 6: return pconst && A->pat_desc;
+    case 6: return stencil_ok(A) || (pconst && A->pat_desc);
     case 7: return A->pn64 != nullptr;
     default: return false;
   }
@@ -1155,6 +1158,7 @@ int launch_variant(const evslcu_mat *A, int v, bool first, bool epi, const doubl
                              e ? ep->nbeta : 0.0, e ? ep->dotv : nullptr, e ? ep->dot_out : nullptr);
     }
     case 6:
+      if (stencil_ok(A)) return stencil_step(A, first, vk, vkm1, out, y, t, ncc, s, mu0, epi ? ep : nullptr);
       if (A->pat_f32)
         return launch_cheb_step(PatCDView<true>{n, A->pat_desc}, n, 0, first, epi, vk, vkm1, out, y, t, ncc, s, mu0,
                                 ep);
@@ -1265,6 +1269,10 @@ int evslcu::chebav_per_degree(const evslcu_mat *A, const double *mu, int deg, do
   const int n = A->n;
   const double t1 = 1.0 / dd, t2 = 2.0 / dd, ncc = -cc;
   double *W[2] = {work, work + n};
+  if (stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == 6)) {
+    const_cast<evslcu_mat *>(A)->cheb_ran = 1;
+    return stencil_chebav(A, mu, deg, cc, dd, v, y, work, epi);
+  }
   const int var = cheb_variant(A);
   if (var == -2) return fail(EVSLCU_ERR_ARG, "filter kernel variant %d is not available for this matrix", g_cheb_force);
   if (var <= EVSLCU_ERR_CUDA) return var;
@@ -1328,6 +1336,9 @@ double evslcu_chebav_step_cost(evslcu_mat *A) {
 
 int evslcu_mat_cheb_variant(const evslcu_mat *A, float *us) {
   if (!A) return fail(EVSLCU_ERR_ARG, "null matrix");
+  // a matrix filtered on its merged stencil has its variants timed when the
+  // times are asked for
+  if (A->cheb_variant < 0 && A->cheb_ran) cheb_variant(A);
   if (us)
     for (int v = 0; v < kChebVariants; ++v) us[v] = A->cheb_us[v];
   return A->cheb_variant;
@@ -1411,7 +1422,7 @@ evslcu_mat *evslcu_mat_create(int n, int nnz, const int *ia, const int *ja, cons
     }
   }
   if (build_sell_device(M, g_compress != 0) || evslcu_sync() || (g_patterns && build_patterns_device(M)) ||
-      pat_const_claim(M)) {
+      pat_const_claim(M) || stencil_build(M)) {
     evslcu_mat_destroy(M);
     return nullptr;
   }
@@ -1438,6 +1449,7 @@ void evslcu_mat_destroy(evslcu_mat *M) {
   evslcu_free(M->wave_mu);
   evslcu_free(M->sval32);
   pat_const_release(M);
+  stencil_free(M);
   evslcu_free(M->pat_id);
   evslcu_free(M->pat_table);
   delete M;

@@ -92,12 +92,21 @@ struct evslcu_mat {
   int pat_cent = -1;   // first entry of the table's copy in the constant pool (-1: not there)
   int pat_chdr = -1;   // first header there
   unsigned *pat_desc = nullptr;  // per row: (first pool entry << 8) | count, when in the pool
+  // Merged stencil of the dictionary (stencil.cuh): st_d entries in increasing
+  // offset order and a mask of them per row; st_d 0: none.
+  int st_d = 0;
+  int st_reach = 0;  // largest |offset|
+  int st_span = 0;   // largest offset: rows r and r + st_span share most of what they gather
+  void *st_mask = nullptr;
+  double st_val[32] = {};
+  int st_off[32] = {};
   int use_pat = 0;     // 1: the FP64 single-vector filter and SpMV read the dictionary
   evslcu_panels *pn64 = nullptr;  // column-panel layout for the FP64 kernels (large general matrices)
   evslcu_panels *pn32 = nullptr;  // the same for the FP32 kernels
   evslcu_xsplit *xs[6] = {};      // column-split copies with 1, 2, 4, 8, 16, 32 ranges (null: not built)
   void *xs_acc = nullptr;         // partial-sum block of the column-split filter (n x 16 doubles)
   int xs_bad = 0;                 // 1: no column-split copy (a row's columns are not increasing)
+  int cheb_ran = 0;           // 1: the single-vector filter has run on the merged stencil
   int cheb_variant = -1;      // single-vector filter kernel chosen by timing (-1: not yet)
   float cheb_us[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // measured time per degree step of each variant
   int cheb_grid = 0;                      // tuned block limit per degree step (0: one row per thread)
@@ -474,6 +483,15 @@ int chebav_per_degree(const evslcu_mat *A, const double *mu, int deg, double cc,
 // Filter through a user matvec callback (sparse.cu).
 int chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, double cc, double dd, const double *v,
                        double *y, double *work, const evslcu_cheb_epi *epi);
+// Merged stencil (stencil.cu): build from the dictionary, whether the filters
+// use it, and the filter on it.
+int stencil_build(evslcu_mat *M);
+void stencil_free(evslcu_mat *M);
+bool stencil_ok(const evslcu_mat *M);
+int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,
+                   double *work, const evslcu_cheb_epi *epi);
+int stencil_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y,
+                 double t, double ncc, double s, double mu0, const evslcu_cheb_epi *epi);
 int launch_scale_copy(int n, double a, const double *x, double *y);
 int launch_lan_epi(int n, const evslcu_cheb_epi *epi, double *y);
 

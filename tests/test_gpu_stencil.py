@@ -1,0 +1,108 @@
+"""The filter on a matrix's merged stencil (stencil.cu) gives the filtered
+vector of the general kernels bit for bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import evsl_b200 as E
+from oracle import evsl_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def stencil_csr(n, entries, drop=0):
+    """CSR of n rows holding `entries` (offset, value) where the column exists;
+    with `drop`, row r leaves out entry (r % drop) when that is not the first."""
+    r = np.arange(n, dtype=np.int64)
+    rows, cols, vals = [], [], []
+    for e, (off, v) in enumerate(sorted(entries)):
+        keep = (r + off >= 0) & (r + off < n)
+        if drop and e > 0:
+            keep &= (r % drop) != e
+        rows.append(r[keep])
+        cols.append(r[keep] + off)
+        vals.append(np.full(int(keep.sum()), v))
+    rows, cols, vals = map(np.concatenate, (rows, cols, vals))
+    order = np.lexsort((cols, rows))
+    ia = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(rows, minlength=n), out=ia[1:])
+    return ia.astype(np.int32), cols[order].astype(np.int32), vals[order]
+
+
+def box9(nx):
+    return [(i + nx * j, 0.1 * i + j + 3.0) for j in (-1, 0, 1) for i in (-1, 0, 1)]
+
+
+def box27(nx, nxy):
+    return [(i + nx * j + nxy * k, 0.01 * (i + 2 * j + 5 * k) + (7.0 if i == j == k == 0 else -0.2))
+            for k in (-1, 0, 1) for j in (-1, 0, 1) for i in (-1, 0, 1)]
+
+
+SHAPES = {
+    # name: (rows, entries, drop); widths 5, 7, 9, 16 and 32, masks of 1, 2 and 4 bytes
+    "one-row": (1, [(0, 2.5)], 0),
+    "tridiagonal": (257, [(-1, -1.0), (0, 2.0), (1, -1.0)], 0),
+    "line-255": (255, [(-40, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (40, -1.0)], 0),
+    "plane-7": (5003, [(-400, -1.0), (-20, -0.5), (-1, -1.0), (0, 6.1), (1, -1.0), (20, -0.5), (400, -1.0)], 0),
+    "dropped-7": (4099, [(-400, -1.0), (-20, -0.5), (-1, -1.0), (0, 6.1), (1, -1.0), (20, -0.5), (400, -1.0)], 7),
+    "lopsided": (3001, [(-7, 0.3), (0, 2.0), (5, 0.7), (90, -0.4)], 0),
+    "no-diagonal": (1000, [(-3, 0.3), (-1, 0.6), (1, 0.6), (3, 0.3)], 0),
+    "box-9": (6007, box9(60), 0),
+    "eleven": (2048, [(o, 0.1 * o + 1.0) for o in range(-5, 6)], 6),
+    "box-27": (9001, box27(20, 400), 0),
+    "thirty-two": (3000, [(o, 1.0 / (40 + o)) for o in range(-16, 16)], 0),
+    # rows past the size where a thread takes two rows an offset apart
+    "two-rows-5": (150001, [(-387, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (387, -1.0)], 0),
+    "two-rows-7": (160003, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
+    "two-rows-dropped": (151000, [(-900, -1.0), (-30, 0.2), (-1, -1.0), (0, 6.0), (1, -1.0), (30, 0.2), (900, -1.0)], 7),
+    "two-rows-9": (155555, box9(400), 0),
+    # the march's stride is more than half the rows: one row per thread again
+    "wide-offset": (150100, [(-80000, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (80000, -1.0)], 0),
+}
+
+
+def polynomial(lib, deg, bound):
+    """A polparams of exactly `deg` with seeded coefficients (and their array)."""
+    pol = E.PolParams()
+    lib.lib.set_pol_def(C.byref(pol))
+    mu = np.random.default_rng(deg).standard_normal(deg + 1)
+    pol.mu = mu.ctypes.data_as(C.POINTER(C.c_double))
+    pol.deg, pol.cc, pol.dd = deg, 0.1 * bound, bound
+    return pol, mu
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_stencil_filter_is_bitwise(gpu_lib, shape):
+    n, entries, drop = SHAPES[shape]
+    ia, ja, a = stencil_csr(n, entries, drop)
+    gpu_lib.set_csr(ia, ja, a)
+    assert gpu_lib.row_pattern_count() > 0
+    v = O.seeded_normal(n, 3)
+    bound = max(np.abs(a).max() * len(entries), 1.0)
+    # degrees 1 to 8: every remainder of the three-degree update of y, at the
+    # first and at a later write
+    for deg in range(1, 9):
+        pol, mu = polynomial(gpu_lib, deg, bound)
+        try:
+            y = gpu_lib.chebav(pol, v)
+            gpu_lib.set_filter_kernel(0)  # SELL storage, pinned to the oracle elsewhere
+            assert np.array_equal(y, gpu_lib.chebav(pol, v)), deg
+        finally:
+            gpu_lib.set_filter_kernel(-1)
+
+
+def test_dictionaries_that_do_not_merge_keep_the_other_kernels(gpu_lib):
+    """More than 32 entries, and rows whose columns do not increase."""
+    wide = stencil_csr(2000, [(o, 1.0 / (50 + o)) for o in range(-20, 21)])
+    ia, ja, a = stencil_csr(2000, [(-30, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (30, -1.0)])
+    ja, a = ja.copy(), a.copy()
+    for r in range(0, 2000, 2):
+        ja[ia[r]:ia[r + 1]] = ja[ia[r]:ia[r + 1]][::-1]
+        a[ia[r]:ia[r + 1]] = a[ia[r]:ia[r + 1]][::-1]
+    for m in (wide, (ia, ja, a)):
+        gpu_lib.set_csr(*m)
+        assert gpu_lib.row_pattern_count() > 0
+        v = O.seeded_normal(2000, 3)
+        pol, mu = polynomial(gpu_lib, 7, 8.0)
+        assert np.array_equal(gpu_lib.chebav(pol, v), O.cheb_av(pol.as_dict(), *m, v))
