@@ -15,6 +15,9 @@ int fail(int code, const char *fmt, ...);
 int check_launch(const char *what);
 void count_launch(uint64_t k = 1);
 int sm_count();
+// After a synchronisation: EVSLCU_ERR_TIMEOUT (once) when a bounded wait of a
+// cluster filter launched before ran out, else 0 (stencil.cu).
+int stencil_error();
 // The device the library was started on (its stream and memory live there).
 int lib_device();
 

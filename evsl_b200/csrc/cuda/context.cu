@@ -185,6 +185,7 @@ int evslcu_finish(void) {
   evslcu_trid_release();
   evslcu_lz_release();
   evslcu_gemm_release();
+  evslcu_stencil_release();
   cudaFree(g_ctx.partials);
   cudaFree(g_ctx.counters);
   cudaFree(g_ctx.scalars);
@@ -201,7 +202,7 @@ int evslcu_finish(void) {
 int evslcu_sync(void) {
   if (!g_ctx.ready) return fail(EVSLCU_ERR_STATE, "library not started (EVSLStart)");
   EVSLCU_CUDA(cudaStreamSynchronize(g_ctx.stream));
-  return 0;
+  return stencil_error();
 }
 
 int evslcu_device_name(int dev, char *buf, int len, int *sm, size_t *mem) {
@@ -270,7 +271,7 @@ int evslcu_d2h(void *dst, const void *src, size_t nbytes) {
   if (!nbytes) return 0;
   EVSLCU_CUDA(cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyDeviceToHost, g_ctx.stream));
   EVSLCU_CUDA(cudaStreamSynchronize(g_ctx.stream));
-  return 0;
+  return stencil_error();
 }
 
 int evslcu_d2d(void *dst, const void *src, size_t nbytes) {

@@ -1249,6 +1249,9 @@ int tune_cheb(evslcu_mat *A) {
 int cheb_variant(const evslcu_mat *A_) {
   evslcu_mat *A = const_cast<evslcu_mat *>(A_);
   if (A->kernel != 0) return -1;
+  // a matrix with a merged stencil claims constant memory only when the
+  // variants that read it are asked for
+  if (A->st_d && A->pat_chdr < 0 && pat_const_claim(A)) return EVSLCU_ERR_CUDA;
   if (g_cheb_force == 7 && panel_candidate(A) && !A->pn64) {
     const int prc = panel_build(A, 0);
     if (prc) return prc;
@@ -1422,7 +1425,7 @@ evslcu_mat *evslcu_mat_create(int n, int nnz, const int *ia, const int *ja, cons
     }
   }
   if (build_sell_device(M, g_compress != 0) || evslcu_sync() || (g_patterns && build_patterns_device(M)) ||
-      pat_const_claim(M) || stencil_build(M)) {
+      stencil_build(M) || (!M->st_d && pat_const_claim(M))) {
     evslcu_mat_destroy(M);
     return nullptr;
   }
@@ -1470,6 +1473,7 @@ int evslcu_mat_get_kernel(const evslcu_mat *A) { return A ? A->kernel : -1; }
 int evslcu_spmv(const evslcu_mat *A, const double *x, double *y) {
   if (!A) return fail(EVSLCU_ERR_ARG, "null matrix");
   const int grid = grid_for(A->n);
+  if (stencil_ok(A)) return stencil_spmv(A, x, y, 1);
   if (evslcu_mat_uses_patterns(A)) {
     if (A->pat_chdr >= 0 && g_pattern_const && A->pat_f32)
       k_spmv<PatCPView><<<grid, kThreads, 0, stream()>>>(PatCPView{A->n, A->pat_id, A->pat_chdr}, x, y);
@@ -1502,6 +1506,11 @@ int evslcu_spmv_cols(const evslcu_mat *A, const double *X, double *Y, int m) {
     const dim3 g(gx, mc);
     const double *Xc = X + (size_t)c0 * ld;
     double *Yc = Y + (size_t)c0 * ld;
+    if (stencil_ok(A)) {
+      const int rc = stencil_spmv(A, Xc, Yc, mc);
+      if (rc) return rc;
+      continue;
+    }
     if (evslcu_mat_uses_patterns(A)) {
       if (A->pat_chdr >= 0 && g_pattern_const && A->pat_f32)
         k_spmv_cols<PatCPView><<<g, kThreads, 0, stream()>>>(PatCPView{A->n, A->pat_id, A->pat_chdr}, Xc, Yc, ld);

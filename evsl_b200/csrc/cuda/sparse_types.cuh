@@ -488,6 +488,7 @@ int chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, double cc
 int stencil_build(evslcu_mat *M);
 void stencil_free(evslcu_mat *M);
 bool stencil_ok(const evslcu_mat *M);
+int stencil_spmv(const evslcu_mat *A, const double *X, double *Y, int m);
 int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,
                    double *work, const evslcu_cheb_epi *epi);
 int stencil_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y,

@@ -77,6 +77,16 @@ inline StArg<VT, D> st_arg(const evslcu_mat *A) {
 // the other filter kernels.
 __device__ __forceinline__ double st_fmadd(double a, double b, double acc) { return __dadd_rn(acc, __dmul_rn(a, b)); }
 __device__ __forceinline__ float st_fmadd(float a, float b, float acc) { return fmaf(a, b, acc); }
+// The zero whose product with v is -0 (v finite).  Adding -0 leaves every sum
+// as it is, signed zeros included, so a row takes an absent entry as v times
+// this zero.
+__device__ __forceinline__ double st_zero(double v) {
+  return __hiloint2double((~__double2hiint(v)) & (int)0x80000000, 0);
+}
+__device__ __forceinline__ float st_zero(float v) { return __uint_as_float(~__float_as_uint(v) & 0x80000000u); }
+// y += c w: rounded multiply and add in both precisions.
+__device__ __forceinline__ double st_fmadd_y(double c, double w, double y) { return __dadd_rn(y, __dmul_rn(c, w)); }
+__device__ __forceinline__ float st_fmadd_y(float c, float w, float y) { return __fadd_rn(y, __fmul_rn(c, w)); }
 __device__ __forceinline__ double st_mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float st_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double st_add(double a, double b) { return __dadd_rn(a, b); }

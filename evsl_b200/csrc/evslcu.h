@@ -355,6 +355,12 @@ int evslcu_scal_batch(int ns, const int *n, double *const *x, const double *a, v
 void evslcu_lz_release(void);
 /* Free the cached split-K partial products of evslcu_dgemm. */
 void evslcu_gemm_release(void);
+/* Frees the stencil filter's device coefficients (EVSLFinish). */
+void evslcu_stencil_release(void);
+/* Blocks per cluster of the single-launch stencil filter (stencil.cu): 0
+ * chosen by size (default), a power of two up to 16, or -1 for one launch per
+ * degree.  Results are identical. */
+int evslcu_set_stencil_cluster(int blocks);
 /* Free the cached KPM and tridiagonal workspaces (evslcu_finish calls them). */
 void evslcu_kpm_release(void);
 void evslcu_trid_release(void);

@@ -52,6 +52,12 @@ SHAPES = {
     "eleven": (2048, [(o, 0.1 * o + 1.0) for o in range(-5, 6)], 6),
     "box-27": (9001, box27(20, 400), 0),
     "thirty-two": (3000, [(o, 1.0 / (40 + o)) for o in range(-16, 16)], 0),
+    # the rows of a cluster's blocks fall on and around their edges
+    "cluster-exact": (16 * 96, [(-96, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (96, -1.0)], 0),
+    "cluster-over": (16 * 96 + 1, [(-96, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (96, -1.0)], 0),
+    "cluster-halo-rows": (700, [(-200, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (200, -1.0)], 0),
+    "cluster-loop": (13000, [(-777, -1.0), (-9, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (9, -1.0), (777, -1.0)], 0),
+    "cluster-y-global": (122000, [(-3300, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (3300, -1.0)], 0),
     # rows past the size where a thread takes two rows an offset apart
     "two-rows-5": (150001, [(-387, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (387, -1.0)], 0),
     "two-rows-7": (160003, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
@@ -72,8 +78,11 @@ def polynomial(lib, deg, bound):
     return pol, mu
 
 
+# one launch per degree, and one cluster of the largest, a middle and the
+# smallest size (stencils too wide or too long for a cluster take the former)
+@pytest.mark.parametrize("blocks", [-1, 0, 4, 1])
 @pytest.mark.parametrize("shape", sorted(SHAPES))
-def test_stencil_filter_is_bitwise(gpu_lib, shape):
+def test_stencil_filter_is_bitwise(gpu_lib, shape, blocks):
     n, entries, drop = SHAPES[shape]
     ia, ja, a = stencil_csr(n, entries, drop)
     gpu_lib.set_csr(ia, ja, a)
@@ -85,11 +94,13 @@ def test_stencil_filter_is_bitwise(gpu_lib, shape):
     for deg in range(1, 9):
         pol, mu = polynomial(gpu_lib, deg, bound)
         try:
+            gpu_lib.lib.evslcu_set_stencil_cluster(blocks)
             y = gpu_lib.chebav(pol, v)
             gpu_lib.set_filter_kernel(0)  # SELL storage, pinned to the oracle elsewhere
             assert np.array_equal(y, gpu_lib.chebav(pol, v)), deg
         finally:
             gpu_lib.set_filter_kernel(-1)
+            gpu_lib.lib.evslcu_set_stencil_cluster(0)
 
 
 def test_dictionaries_that_do_not_merge_keep_the_other_kernels(gpu_lib):
