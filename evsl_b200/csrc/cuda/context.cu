@@ -186,6 +186,7 @@ int evslcu_finish(void) {
   evslcu_lz_release();
   evslcu_gemm_release();
   evslcu_stencil_release();
+  evslcu_lan_release();
   cudaFree(g_ctx.partials);
   cudaFree(g_ctx.counters);
   cudaFree(g_ctx.scalars);

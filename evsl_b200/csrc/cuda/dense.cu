@@ -58,7 +58,7 @@ __global__ void k_scal(int n, double a, double *x) {
 // [2] done flag (1.0 once the DGKS test has passed).
 // ---------------------------------------------------------------------------
 constexpr int kGemvTRows = 1024;   // rows per chunk of the transposed product
-constexpr int kGemvTCols = 32;     // columns per block
+constexpr int kGemvTCols = 32;     // most columns per block
 constexpr int kGemvNChunk = 2048;  // h values staged in shared memory at once
 
 // part[chunk * k + j] = sum over the chunk's rows of Q[r, j] * v[r]; block
@@ -66,14 +66,14 @@ constexpr int kGemvNChunk = 2048;  // h values staged in shared memory at once
 // kernel and the engine's batched one, so both round alike.
 __device__ __forceinline__ void gemvT_partial_body(int n, int k, const double *__restrict__ Q, long long ld,
                                                    const double *__restrict__ v, double *__restrict__ part, int bx,
-                                                   int by, double *sv) {
+                                                   int by, int cols, double *sv) {
   const int r0 = bx * kGemvTRows;
   const int rows = min(kGemvTRows, n - r0);
   for (int i = threadIdx.x; i < kGemvTRows; i += blockDim.x) sv[i] = (i < rows) ? v[r0 + i] : 0.0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int jj = warp; jj < kGemvTCols; jj += kThreads / 32) {
-    const int j = by * kGemvTCols + jj;
+  for (int jj = warp; jj < cols; jj += kThreads / 32) {
+    const int j = by * cols + jj;
     if (j >= k) break;
     const double *q = Q + (long long)j * ld + r0;
     double acc = 0.0;
@@ -84,12 +84,14 @@ __device__ __forceinline__ void gemvT_partial_body(int n, int k, const double *_
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
-    k_gemvT_partial(int n, int k, const double *__restrict__ Q, long long ld, const double *__restrict__ v,
-                    double *__restrict__ part, const double *state) {
-  if (state && state[2] != 0.0) return;
-  __shared__ double sv[kGemvTRows];
-  gemvT_partial_body(n, k, Q, ld, v, part, blockIdx.x, blockIdx.y, sv);
+// Columns a block of the transposed product takes (one warp each, or two or
+// four one after another): few when the product is small, so that every SM has
+// blocks.  A column's sum does not depend on it.
+inline int gemvT_cols(int nchunks, int k) {
+  const long long fill = 4LL * sm_count();
+  for (int c = kGemvTCols; c > 8; c /= 2)
+    if ((long long)nchunks * ((k + c - 1) / c) >= fill) return c;
+  return 8;
 }
 
 // h[j] = alpha * sum_chunks part[chunk*k + j] (+ beta * h[j] when beta != 0).
@@ -120,18 +122,70 @@ __global__ void __launch_bounds__(256)
   gemvT_reduce_body(nchunks, k, part, alpha, beta, h, blockIdx.x, sh);
 }
 
-// v[r] <- v[r] + sum_j (alpha*h[j]) * Q[r, j], summed over j in order as the
-// reference dgemv('N') does.  With `state`, also computes ||v|| and applies
-// the DGKS decision of SRC/misc_la.c:246-250.
-// Rows bx*blockDim.x + threadIdx.x + i*gx*blockDim.x of the update; returns
-// this thread's sum of the new z^2.
+// Blocks of a column tile that have finished (k_gemvT), zero between kernels.
+constexpr int kTileCtrs = 4096;
+__device__ unsigned g_tile_ctr[kTileCtrs];
+
+// The transposed product's partial sums; with `reduce`, the last block of each
+// column tile also sums its columns over the chunks (gemvT_reduce_body's
+// order) into h = alpha V^T v: one launch instead of two.
+__global__ void __launch_bounds__(kThreads)
+    k_gemvT(int n, int k, const double *__restrict__ Q, long long ld, const double *__restrict__ v, double *part,
+            int cols, int reduce, double alpha, double *h, const double *state) {
+  if (state && state[2] != 0.0) return;
+  __shared__ double sv[kGemvTRows];
+  __shared__ double sh[8][33];
+  __shared__ bool last;
+  gemvT_partial_body(n, k, Q, ld, v, part, blockIdx.x, blockIdx.y, cols, sv);
+  if (!reduce) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(g_tile_ctr + blockIdx.y, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nchunks = gridDim.x;
+  const int j = blockIdx.y * cols + lane;
+  const bool on = lane < cols && j < k;
+  double s = 0.0;
+  if (on)
+    for (int c = warp; c < nchunks; c += 8) s += __ldcg(part + (long long)c * k + j);
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && on) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += sh[w][lane];
+    h[j] = alpha * t;
+  }
+  if (threadIdx.x == 0) g_tile_ctr[blockIdx.y] = 0u;
+}
+
+// Column groups of the product V h: a block of 256 threads takes 256 / G rows,
+// and its G groups of threads every G-th column of them.  With one thread per
+// row (G = 1) a row's k columns are one chain of load batches, and below about
+// 10^5 rows most SMs have no block at all.  A function of n alone, so that a
+// vector is orthogonalised alike wherever it is done.
+inline int gemvN_groups(int n) { return n <= 40000 ? 8 : n <= 80000 ? 4 : n <= 160000 ? 2 : 1; }
+inline int gemvN_grid(int n) { return grid_for(n, kThreads / gemvN_groups(n), kMaxPartials); }
+
+// v[r] <- v[r] + sum_j (alpha*h[j]) * Q[r, j]: one group adds the columns to
+// v[r] in order, as the reference dgemv('N') does; several groups sum their
+// columns in order, and the groups' sums are added in order and then to v[r].
+// With `state`, also computes ||v|| and applies the DGKS decision of
+// SRC/misc_la.c:246-250.  Block bx of gx; returns this thread's sum of the new
+// z^2.  sh_h: kGemvNChunk doubles.
+template <int G>
 __device__ __forceinline__ double gemvN_body(int n, int k, const double *__restrict__ Q, long long ld,
                                              const double *__restrict__ h, double alpha, double *v, int bx, int gx,
                                              double *sh_h) {
+  constexpr int RB = kThreads / G;
+  const int lr = threadIdx.x % RB, grp = threadIdx.x / RB;
   double nsum = 0.0;
-  for (long long base = (long long)bx * blockDim.x; base < n; base += (long long)gx * blockDim.x) {
-    const long long r = base + threadIdx.x;
-    double z = (r < n) ? v[r] : 0.0;
+  for (long long base = (long long)bx * RB; base < n; base += (long long)gx * RB) {
+    const long long r = base + lr;
+    double z = (r < n && grp == 0) ? v[r] : 0.0;
+    double acc = G == 1 ? z : 0.0;
     for (int j0 = 0; j0 < k; j0 += kGemvNChunk) {
       const int cnt = min(kGemvNChunk, k - j0);
       __syncthreads();
@@ -139,20 +193,33 @@ __device__ __forceinline__ double gemvN_body(int n, int k, const double *__restr
       __syncthreads();
       if (r < n) {
         // 16 column loads in flight per thread, then the updates in column
-        // order (the summation order is unchanged)
+        // order
         const double *q = Q + (long long)j0 * ld + r;
-        int j = 0;
-        for (; j + 16 <= cnt; j += 16) {
+        int j = grp;
+        for (; j + 15 * G < cnt; j += 16 * G) {
           double x[16];
 #pragma unroll
-          for (int u = 0; u < 16; ++u) x[u] = __ldg(q + (long long)(j + u) * ld);
+          for (int u = 0; u < 16; ++u) x[u] = __ldg(q + (long long)(j + u * G) * ld);
 #pragma unroll
-          for (int u = 0; u < 16; ++u) z = __dadd_rn(z, __dmul_rn(sh_h[j + u], x[u]));
+          for (int u = 0; u < 16; ++u) acc = __dadd_rn(acc, __dmul_rn(sh_h[j + u * G], x[u]));
         }
-        for (; j < cnt; ++j) z = __dadd_rn(z, __dmul_rn(sh_h[j], __ldg(q + (long long)j * ld)));
+        for (; j < cnt; j += G) acc = __dadd_rn(acc, __dmul_rn(sh_h[j], __ldg(q + (long long)j * ld)));
       }
     }
-    if (r < n) {
+    if (G == 1) {
+      z = acc;
+    } else {
+      __syncthreads();
+      sh_h[threadIdx.x] = acc;
+      __syncthreads();
+      if (grp == 0) {
+        double t = acc;
+#pragma unroll
+        for (int g = 1; g < G; ++g) t += sh_h[g * RB + lr];
+        z = __dadd_rn(z, t);
+      }
+    }
+    if (r < n && grp == 0) {
       v[r] = z;
       nsum += z * z;
     }
@@ -170,30 +237,94 @@ __device__ __forceinline__ void dgks_decide(double t, double *state) {
     state[0] = nw;
 }
 
+// out (optional): the norm; host (optional, mapped): alpha, the norm and
+// whether the DGKS test has passed, for the solver that waits for them.
+template <int G>
 __global__ void __launch_bounds__(kThreads)
     k_gemvN(int n, int k, const double *__restrict__ Q, long long ld, const double *__restrict__ h, double alpha,
-            double *v, double *part, unsigned int *ctr, double *state) {
+            double *v, double *part, unsigned int *ctr, double *state, double *out, const double *d_alpha,
+            double *host) {
   if (state && state[2] != 0.0) return;
   __shared__ double sh_h[kGemvNChunk];
   __shared__ double sh[kThreads / 32];
-  double nsum = gemvN_body(n, k, Q, ld, h, alpha, v, blockIdx.x, gridDim.x, sh_h);
+  double nsum = gemvN_body<G>(n, k, Q, ld, h, alpha, v, blockIdx.x, gridDim.x, sh_h);
   if (state) {
     nsum = block_sum(nsum, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = nsum;
     if (last_block(ctr)) {
       double t = reduce_partials(part, gridDim.x, ctr, sh);
-      if (threadIdx.x == 0) dgks_decide(t, state);
+      if (threadIdx.x == 0) {
+        dgks_decide(t, state);
+        if (out) *out = state[1];
+        if (host) {
+          host[0] = *d_alpha;
+          host[1] = state[1];
+          host[2] = state[2];
+        }
+      }
     }
   }
 }
 
-__global__ void k_cgs_init(double *state, const double *nrm) {
-  state[0] = *nrm;
-  state[1] = 0.0;
-  state[2] = 0.0;
+int launch_gemvN(int n, int k, const double *Q, long long ld, const double *h, double alpha, double *v, double *state,
+                 double *out, const double *d_alpha, double *host) {
+  const int g = gemvN_grid(n);
+  double *part = state ? partials() : nullptr;
+  unsigned int *ctr = state ? counters() + CTR_CGS : nullptr;
+  auto fn = k_gemvN<1>;
+  switch (gemvN_groups(n)) {
+    case 8: fn = k_gemvN<8>; break;
+    case 4: fn = k_gemvN<4>; break;
+    case 2: fn = k_gemvN<2>; break;
+    default: break;
+  }
+  fn<<<g, kThreads, 0, stream()>>>(n, k, Q, ld, h, alpha, v, part, ctr, state, out, d_alpha, host);
+  EVSLCU_LAUNCH_CHECK("k_gemvN");
+  return 0;
 }
 
-__global__ void k_copy_scalar(const double *src, double *dst) { *dst = *src; }
+// h = alpha Q^T v through `part` (chunks x k partial sums).
+int launch_gemvT(int n, int k, const double *Q, long long ld, const double *v, double *part, double alpha, double *h,
+                 const double *state) {
+  const int nchunks = (n + kGemvTRows - 1) / kGemvTRows;
+  const int cols = gemvT_cols(nchunks, k), tiles = (k + cols - 1) / cols;
+  const int reduce = tiles <= kTileCtrs ? 1 : 0;
+  k_gemvT<<<dim3(nchunks, tiles), kThreads, 0, stream()>>>(n, k, Q, ld, v, part, cols, reduce, alpha, h, state);
+  EVSLCU_LAUNCH_CHECK("k_gemvT");
+  if (!reduce) {
+    k_gemvT_reduce<<<(k + 31) / 32, 256, 0, stream()>>>(nchunks, k, part, alpha, 0.0, h, state);
+    EVSLCU_LAUNCH_CHECK("k_gemvT_reduce");
+  }
+  return 0;
+}
+
+// Starting norm of the Gram-Schmidt passes, ||y|| after y += sign coef x (when
+// x is given): k_axpy_ds, the norm of k_dot and the passes' state in one.
+__global__ void __launch_bounds__(kThreads)
+    k_cgs_start(int n, const double *coef, double sign, const double *x, double *y, double *part, unsigned int *ctr,
+                double *state) {
+  __shared__ double sh[kThreads / 32];
+  const double c = x ? sign * (*coef) : 0.0;
+  double s = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double yi = y[i];
+    if (x) {
+      yi = __dadd_rn(yi, __dmul_rn(c, x[i]));
+      y[i] = yi;
+    }
+    s += yi * yi;
+  }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  if (last_block(ctr)) {
+    const double t = reduce_partials(part, gridDim.x, ctr, sh);
+    if (threadIdx.x == 0) {
+      state[0] = sqrt(t);
+      state[1] = 0.0;
+      state[2] = 0.0;
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // The request engine's Lanczos step for many slots at once.  Every slot's
@@ -209,6 +340,7 @@ struct LzSlot {
   int n, kc;            // rows; basis columns orthogonalised against (k + 1)
   int g_dot, nchunks;   // grids of the dot / norm and of the transposed GEMV
   int ctiles, g_n;      // column tiles of the transposed GEMV; grid of the GEMV
+  int tcols, groups;    // columns per tile; column groups of the GEMV
   double nbeta;         // -beta of the previous step (0 at k = 0: no update)
   const double *V;      // basis, ld = n
   const double *v;      // V(:, k)
@@ -280,7 +412,7 @@ __global__ void __launch_bounds__(kThreads) k_lz_axpy_nrm(const LzSlot *__restri
   if (threadIdx.x == 0) S.npart[b] = acc;
 }
 
-// the starting norm of the Gram-Schmidt passes (k_cgs_init)
+// the starting norm of the Gram-Schmidt passes (k_cgs_start)
 __global__ void __launch_bounds__(kThreads) k_lz_cgs_init(const LzSlot *__restrict__ SS) {
   __shared__ double sh[kThreads / 32];
   const LzSlot &S = SS[blockIdx.x];
@@ -302,7 +434,7 @@ __global__ void __launch_bounds__(kThreads) k_lz_gemvT(const LzSlot *__restrict_
   const LzSlot &S = SS[si];
   if (lz_state(S)[2] != 0.0) return;
   const int b = blockIdx.x - pre[si];
-  gemvT_partial_body(S.n, S.kc, S.V, S.n, S.z, S.part, b % S.nchunks, b / S.nchunks, sv);
+  gemvT_partial_body(S.n, S.kc, S.V, S.n, S.z, S.part, b % S.nchunks, b / S.nchunks, S.tcols, sv);
 }
 
 __global__ void __launch_bounds__(256) k_lz_gemvT_reduce(const LzSlot *__restrict__ SS, const int *__restrict__ pre,
@@ -322,7 +454,13 @@ __global__ void __launch_bounds__(kThreads) k_lz_gemvN(const LzSlot *__restrict_
   const LzSlot &S = SS[si];
   if (lz_state(S)[2] != 0.0) return;
   const int b = blockIdx.x - pre[si];
-  double nsum = gemvN_body(S.n, S.kc, S.V, S.n, lz_h(S), -1.0, S.z, b, S.g_n, sh_h);
+  double nsum;
+  switch (S.groups) {
+    case 8: nsum = gemvN_body<8>(S.n, S.kc, S.V, S.n, lz_h(S), -1.0, S.z, b, S.g_n, sh_h); break;
+    case 4: nsum = gemvN_body<4>(S.n, S.kc, S.V, S.n, lz_h(S), -1.0, S.z, b, S.g_n, sh_h); break;
+    case 2: nsum = gemvN_body<2>(S.n, S.kc, S.V, S.n, lz_h(S), -1.0, S.z, b, S.g_n, sh_h); break;
+    default: nsum = gemvN_body<1>(S.n, S.kc, S.V, S.n, lz_h(S), -1.0, S.z, b, S.g_n, sh_h); break;
+  }
   nsum = block_sum(nsum, sh);
   if (threadIdx.x == 0) S.npart[b] = nsum;
 }
@@ -833,8 +971,10 @@ int evslcu_lanczos_batch(int ns, const evslcu_lz_col *cols, int imax, void *tabl
     L.kc = c.k + 1;
     L.g_dot = grid_for(c.n, kThreads, 1024);
     L.nchunks = (c.n + kGemvTRows - 1) / kGemvTRows;
-    L.ctiles = (L.kc + kGemvTCols - 1) / kGemvTCols;
-    L.g_n = grid_for(c.n, kThreads, kMaxPartials);
+    L.tcols = gemvT_cols(L.nchunks, L.kc);
+    L.ctiles = (L.kc + L.tcols - 1) / L.tcols;
+    L.g_n = gemvN_grid(c.n);
+    L.groups = gemvN_groups(c.n);
     L.nbeta = -c.beta;
     L.V = c.V;
     L.v = c.V + (size_t)c.k * c.n;
@@ -940,33 +1080,66 @@ int evslcu_block_cgs2(int n, int m, double *W, int b, double *H, double *norm_de
   return rc;
 }
 
+// Scalars of a Lanczos step that the host waits for: written by the step's
+// last kernel straight into pinned host memory, read after a synchronisation.
+static double *g_lan_host = nullptr;
+
+void evslcu_lan_release(void) {
+  if (g_lan_host) cudaFreeHost(g_lan_host);
+  g_lan_host = nullptr;
+}
+
+// One Gram-Schmidt pass of v against Q(:, 0:k): two launches.
+static int cgs_pass(int n, int k, const double *Q, long long ldq, double *v, double *part, double *h, double *state,
+                    double *out, const double *d_alpha, double *host) {
+  const int rc = launch_gemvT(n, k, Q, ldq, v, part, 1.0, h, state);
+  return rc ? rc : launch_gemvN(n, k, Q, ldq, h, -1.0, v, state, out, d_alpha, host);
+}
+
+static int cgs_start(int n, const double *coef, double sign, const double *x, double *v, double *state) {
+  k_cgs_start<<<grid_for(n, kThreads, 1024), kThreads, 0, stream()>>>(n, coef, sign, x, v, partials(),
+                                                                      counters() + CTR_NRM, state);
+  EVSLCU_LAUNCH_CHECK("k_cgs_start");
+  return 0;
+}
+
 int evslcu_cgs_dgks(int n, int k, int imax, const double *Q, long long ldq, double *v, double *nrm_out_dev,
                     double *work) {
   if (k < 1 || n < 1) return fail(EVSLCU_ERR_ARG, "cgs: bad sizes n=%d k=%d", n, k);
   const int nchunks = (n + kGemvTRows - 1) / kGemvTRows;
-  double *part = work;
-  double *h = work + (size_t)nchunks * k;
-  double *state = h + k;
-  double *nrm0 = state + 4;
-  cudaStream_t st = stream();
-  int rc;
-  if ((rc = evslcu_nrm2(n, v, nrm0))) return rc;
-  k_cgs_init<<<1, 1, 0, st>>>(state, nrm0);
-  EVSLCU_LAUNCH_CHECK("k_cgs_init");
-  const dim3 gT(nchunks, (k + kGemvTCols - 1) / kGemvTCols);
-  const int gN = grid_for(n, kThreads, kMaxPartials);
-  for (int pass = 0; pass < imax; ++pass) {
-    k_gemvT_partial<<<gT, kThreads, 0, st>>>(n, k, Q, ldq, v, part, state);
-    EVSLCU_LAUNCH_CHECK("k_gemvT_partial");
-    k_gemvT_reduce<<<(k + 31) / 32, 256, 0, st>>>(nchunks, k, part, 1.0, 0.0, h, state);
-    EVSLCU_LAUNCH_CHECK("k_gemvT_reduce");
-    k_gemvN<<<gN, kThreads, 0, st>>>(n, k, Q, ldq, h, -1.0, v, partials(), counters() + CTR_CGS, state);
-    EVSLCU_LAUNCH_CHECK("k_gemvN");
+  double *part = work, *h = work + (size_t)nchunks * k, *state = h + k;
+  int rc = cgs_start(n, nullptr, 0.0, nullptr, v, state);
+  for (int pass = 0; !rc && pass < imax; ++pass)
+    rc = cgs_pass(n, k, Q, ldq, v, part, h, state, nrm_out_dev, nullptr, nullptr);
+  return rc;
+}
+
+// The end of a Lanczos step: z -= alpha v, z orthogonalised against V(:, 0:k)
+// by classical Gram-Schmidt with the DGKS test (evslcu_cgs_dgks), alpha and
+// beta = ||z|| returned to the host.  The host waits for them anyway, so it is
+// the host that starts a second pass, when the first has not passed the test:
+// three launches for nearly every step.
+int evslcu_lan_orth(int n, int k, int imax, const double *V, long long ldv, const double *d_alpha, const double *v,
+                    double *z, double *work, evslcu_marks *marks, int mark, double *alpha, double *beta) {
+  if (k < 1 || n < 1) return fail(EVSLCU_ERR_ARG, "lan_orth: bad sizes n=%d k=%d", n, k);
+  if (!g_lan_host) {
+    void *p = nullptr;
+    EVSLCU_CUDA(cudaHostAlloc(&p, 4 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
+    g_lan_host = (double *)p;
   }
-  if (nrm_out_dev) {
-    k_copy_scalar<<<1, 1, 0, st>>>(state + 1, nrm_out_dev);
-    EVSLCU_LAUNCH_CHECK("k_copy_scalar");
+  const int nchunks = (n + kGemvTRows - 1) / kGemvTRows;
+  double *part = work, *h = work + (size_t)nchunks * k, *state = h + k;
+  volatile double *got = g_lan_host;
+  int rc = cgs_start(n, d_alpha, -1.0, v, z, state);
+  for (int pass = 0; !rc && pass < imax; ++pass) {
+    rc = cgs_pass(n, k, V, ldv, z, part, h, state, nullptr, d_alpha, g_lan_host);
+    if (!rc && marks) evslcu_marks_record(marks, mark);
+    if (!rc) rc = evslcu_sync();
+    if (!rc && got[2] != 0.0) break;
   }
+  if (rc) return rc;
+  *alpha = got[0];
+  *beta = got[1];
   return 0;
 }
 
@@ -980,10 +1153,11 @@ int evslcu_dgemv(char trans, int m, int n, double alpha, const double *A, long l
     const int nchunks = (m + kGemvTRows - 1) / kGemvTRows;
     double *part = (double *)evslcu_malloc(sizeof(double) * (size_t)nchunks * n);
     if (!part) return EVSLCU_ERR_NOMEM;
-    const dim3 gT(nchunks, (n + kGemvTCols - 1) / kGemvTCols);
-    k_gemvT_partial<<<gT, kThreads, 0, st>>>(m, n, A, lda, x, part, nullptr);
+    const int cols = gemvT_cols(nchunks, n);
+    k_gemvT<<<dim3(nchunks, (n + cols - 1) / cols), kThreads, 0, st>>>(m, n, A, lda, x, part, cols, 0, 1.0, nullptr,
+                                                                      nullptr);
     count_launch();
-    int rc = check_launch("k_gemvT_partial");
+    int rc = check_launch("k_gemvT");
     if (!rc) {
       k_gemvT_reduce<<<(n + 31) / 32, 256, 0, st>>>(nchunks, n, part, alpha, beta, y, nullptr);
       count_launch();
@@ -997,10 +1171,7 @@ int evslcu_dgemv(char trans, int m, int n, double alpha, const double *A, long l
     k_scale_vec<<<grid_for(m), kThreads, 0, st>>>(m, beta, y);
     EVSLCU_LAUNCH_CHECK("k_scale_vec");
   }
-  k_gemvN<<<grid_for(m, kThreads, kMaxPartials), kThreads, 0, st>>>(m, n, A, lda, x, alpha, y, nullptr, nullptr,
-                                                                      nullptr);
-  EVSLCU_LAUNCH_CHECK("k_gemvN");
-  return 0;
+  return launch_gemvN(m, n, A, lda, x, alpha, y, nullptr, nullptr, nullptr, nullptr);
 }
 
 // FP64 throughput probe (the roofline's FP64 peak): chains of FMA on each

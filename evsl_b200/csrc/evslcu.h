@@ -344,6 +344,13 @@ typedef struct {
 size_t evslcu_lz_scratch_doubles(void);
 size_t evslcu_lanczos_batch_table_bytes(int ns);
 int evslcu_lanczos_batch(int ns, const evslcu_lz_col *cols, int imax, void *table, size_t table_bytes);
+/* The end of a Lanczos step: z -= alpha v (alpha on the device), z
+ * orthogonalised against the k columns of V as evslcu_cgs_dgks does, alpha and
+ * ||z|| returned to the host; synchronous.  marks: event `mark` is recorded
+ * after the passes (may be null).  work: evslcu_cgs_work_size(n, k) doubles. */
+int evslcu_lan_orth(int n, int k, int imax, const double *V, long long ldv, const double *d_alpha, const double *v,
+                    double *z, double *work, evslcu_marks *marks, int mark, double *alpha, double *beta);
+void evslcu_lan_release(void);
 /* Block Gram-Schmidt, twice, on the m columns of W (n x m, ld n), blocks of
  * b columns: GEMM projections against the earlier columns, then CGS with the
  * DGKS test and unit norms inside the block.  H: (m - b) x b device doubles;

@@ -132,12 +132,9 @@ int ChebLanNr(double *intv, int maxit, double tol, double *vinit, polparams *pol
     if ((rc = evslcu_chebav(op, pol->mu, deg, pol->cc, pol->dd, v, vnew, wk, &epi))) goto cuda_fail;
     evslstat.n_polAv++;
     evslcu_marks_record(marks, 1);
-    /* znew -= alpha v */
-    if ((rc = evslcu_axpy_ds(n, d_alpha, -1.0, v, vnew))) goto cuda_fail;
-    /* full reorthogonalisation, beta = ||vnew|| */
-    if ((rc = evslcu_cgs_dgks(n, k + 1, EVSL_NGS_MAX, V, (long long)n, vnew, d_beta, cgsw))) goto cuda_fail;
-    evslcu_marks_record(marks, 2);
-    if ((rc = evslcu_get_scalars(ds, h, 2))) goto cuda_fail;
+    /* znew -= alpha v, full reorthogonalisation, beta = ||vnew|| */
+    if ((rc = evslcu_lan_orth(n, k + 1, EVSL_NGS_MAX, V, (long long)n, d_alpha, v, vnew, cgsw, marks, 2, &h[0], &h[1])))
+      goto cuda_fail;
     if (marks) {
       evslstat.t_polAv += evslcu_marks_elapsed(marks, 0, 1);
       evslstat.t_reorth += evslcu_marks_elapsed(marks, 1, 2);

@@ -169,9 +169,8 @@ int ChebLanTr(int lanm, int nev, double *intv, int maxit, double tol, double *vi
         if ((rc = evslcu_chebav(op, pol->mu, deg, pol->cc, pol->dd, v, vnew, work, &epi))) goto cuda_fail;
       }
       it++;
-      if ((rc = evslcu_axpy_ds(n, d_alpha, -1.0, v, vnew))) goto cuda_fail;
-      if ((rc = evslcu_cgs_dgks(n, k, EVSL_NGS_MAX, V, (long long)n, vnew, d_beta, cgsw))) goto cuda_fail;
-      if ((rc = evslcu_get_scalars(ds, h, 2))) goto cuda_fail;
+      if ((rc = evslcu_lan_orth(n, k, EVSL_NGS_MAX, V, (long long)n, d_alpha, v, vnew, cgsw, NULL, 0, &h[0], &h[1])))
+        goto cuda_fail;
       const double alpha = h[0];
       beta = h[1];
       T[(k - 1) * lanm1_l + (k - 1)] = alpha;

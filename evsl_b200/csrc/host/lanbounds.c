@@ -171,9 +171,9 @@ int LanTrbounds(int lanm, int maxit, double tol, double *vinit, int bndtype, dou
       if ((rc = evsl_apply_A(v, vnew))) goto done;
       it++;
       if (zold && (rc = evslcu_axpy(n, -beta, zold, vnew))) goto cuda_fail;
-      if ((rc = evslcu_dot(n, v, vnew, d_alpha)) || (rc = evslcu_axpy_ds(n, d_alpha, -1.0, v, vnew))) goto cuda_fail;
-      if ((rc = evslcu_cgs_dgks(n, k, EVSL_NGS_MAX, V, (long long)n, vnew, d_beta, cgsw))) goto cuda_fail;
-      if ((rc = evslcu_get_scalars(ds, h, 2))) goto cuda_fail;
+      if ((rc = evslcu_dot(n, v, vnew, d_alpha)) ||
+          (rc = evslcu_lan_orth(n, k, EVSL_NGS_MAX, V, (long long)n, d_alpha, v, vnew, cgsw, NULL, 0, &h[0], &h[1])))
+        goto cuda_fail;
       const double alpha = h[0];
       beta = h[1];
       T[(k - 1) * lanm1_l + (k - 1)] = alpha;
