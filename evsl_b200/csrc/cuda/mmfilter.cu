@@ -268,9 +268,30 @@ int evslcu_set_batch_persistent(int on) {
   return 0;
 }
 
+static int filter_batch_degrees(int ncols, const evslcu_batch_col *cols, void *table, size_t table_bytes);
+
 int evslcu_filter_batch(int ncols, const evslcu_batch_col *cols, void *table, size_t table_bytes) {
   if (ncols <= 0) return 0;
   if (!cols || !table) return fail(EVSLCU_ERR_ARG, "filter_batch: bad arguments");
+  for (int i = 0; i < ncols; ++i) {
+    const evslcu_batch_col &c = cols[i];
+    if (!c.A || !c.mu || !c.x || !c.y || !c.w || c.deg < 0 || c.dd == 0.0)
+      return fail(EVSLCU_ERR_ARG, "filter_batch: bad column %d", i);
+  }
+  if (g_mm_persistent) return filter_batch_degrees(ncols, cols, table, table_bytes);
+  // operators that fit a thread-block cluster: every degree of all of them in
+  // one launch (stencil.cu); the others together, one launch per degree
+  std::vector<unsigned char> done((size_t)ncols, 0);
+  const int rc = stencil_batch(ncols, cols, done.data());
+  if (rc) return rc;
+  std::vector<evslcu_batch_col> rest;
+  for (int i = 0; i < ncols; ++i)
+    if (!done[i]) rest.push_back(cols[i]);
+  return filter_batch_degrees((int)rest.size(), rest.data(), table, table_bytes);
+}
+
+static int filter_batch_degrees(int ncols, const evslcu_batch_col *cols, void *table, size_t table_bytes) {
+  if (ncols <= 0) return 0;
   std::vector<int> order(ncols);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return cols[p].deg > cols[q].deg; });
@@ -279,8 +300,6 @@ int evslcu_filter_batch(int ncols, const evslcu_batch_col *cols, void *table, si
   long long rows = 0;
   for (int i = 0; i < ncols; ++i) {
     const evslcu_batch_col &c = cols[order[i]];
-    if (!c.A || !c.mu || !c.x || !c.y || !c.w || c.deg < 0 || c.dd == 0.0)
-      return fail(EVSLCU_ERR_ARG, "filter_batch: bad column %d", order[i]);
     const int n = c.A->n;
     MMItem &I = items[i];
     I.cptr = c.A->cptr;

@@ -17,6 +17,7 @@
 // final and is not written again.
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "common.cuh"
 #include "sparse_types.cuh"
@@ -995,6 +996,11 @@ struct evslcu_filter_plan {
   const double **tab_dev;
   const double **tab_host;
   cudaGraphExec_t exec;
+  // a merged stencil's columns need no graph: few launches, and the vectors'
+  // addresses are kernel arguments
+  double *st_mu;
+  evslcu_filter_col *st_cols;
+  size_t *st_off;
 };
 
 extern "C" {
@@ -1006,6 +1012,14 @@ int evslcu_filter_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu
   if (rc) return rc;
   if (!work || work_bytes < evslcu_filter_columns_work(A->n, fp32, ncols))
     return fail(EVSLCU_ERR_ARG, "filter_columns: work too small");
+  if (g_mf_variant < 0 && stencil_columns_ok(A, ncols, cols)) {
+    std::vector<size_t> off((size_t)ncols);
+    double *mu = stencil_columns_mu(ncols, cols, off.data(), &rc);
+    if (!rc) rc = stencil_columns(A, fp32, ncols, cols, mu, off.data(), work);
+    evslcu_free(mu);
+    const_cast<evslcu_mat *>(A)->mf_ran[fp32 ? 1 : 0][log2_width(group_width(std::min(ncols, kMaxB)))] = 1;
+    return rc;
+  }
   const size_t tabb = 2 * sizeof(double *) * (size_t)ncols;
   const size_t tab_off = work_bytes - (tabb + 255) / 256 * 256;
   const double **tab = (const double **)((char *)work + tab_off);
@@ -1044,6 +1058,20 @@ evslcu_filter_plan *evslcu_filter_plan_create(const evslcu_mat *A, int fp32, int
     evslcu_filter_plan_destroy(P);
     return nullptr;
   }
+  if (g_mf_variant < 0 && stencil_columns_ok(A, ncols, cols)) {
+    int err = 0;
+    P->st_cols = (evslcu_filter_col *)malloc(sizeof(evslcu_filter_col) * (size_t)ncols);
+    P->st_off = (size_t *)malloc(sizeof(size_t) * (size_t)ncols);
+    if (P->st_cols && P->st_off) {
+      memcpy(P->st_cols, cols, sizeof(evslcu_filter_col) * (size_t)ncols);
+      P->st_mu = stencil_columns_mu(ncols, cols, P->st_off, &err);
+    }
+    if (!P->st_mu) {
+      evslcu_filter_plan_destroy(P);
+      return nullptr;
+    }
+    return P;
+  }
   int err = autotune_groups(A, fp32, ncols);
   P->coef = err ? nullptr : coef_build(fp32, ncols, cols, &err);
   if (!P->coef) {
@@ -1077,6 +1105,13 @@ evslcu_filter_plan *evslcu_filter_plan_create(const evslcu_mat *A, int fp32, int
 
 int evslcu_filter_plan_run(evslcu_filter_plan *P, const double *const *x, double *const *y) {
   if (!P || !x || !y) return fail(EVSLCU_ERR_ARG, "filter plan: bad arguments");
+  if (P->st_mu) {
+    for (int c = 0; c < P->ncols; ++c) {
+      P->st_cols[c].x = x[c];
+      P->st_cols[c].y = y[c];
+    }
+    return stencil_columns(P->A, P->fp32, P->ncols, P->st_cols, P->st_mu, P->st_off, P->work);
+  }
   for (int c = 0; c < P->ncols; ++c) {
     P->tab_host[c] = x[c];
     P->tab_host[P->ncols + c] = y[c];
@@ -1106,12 +1141,17 @@ int evslcu_set_xs_range_bytes(long long bytes) {
 }
 
 int evslcu_mat_filter_variant(const evslcu_mat *A, int fp32, int B) {
-  return A ? A->mf_variant[fp32 ? 1 : 0][log2_width(B)] : -1;
+  if (!A) return -1;
+  const int f = fp32 ? 1 : 0, b = log2_width(B);
+  // columns filtered on a merged stencil: the variants are timed when asked for
+  if (A->mf_variant[f][b] < 0 && A->mf_ran[f][b]) autotune(const_cast<evslcu_mat *>(A), fp32, group_width(std::min(B, kMaxB)));
+  return A->mf_variant[f][b];
 }
 
 double evslcu_filter_step_cost(evslcu_mat *A, int fp32, int B) {
   if (!A || A->kernel != 0 || B < 1) return -1.0;
   if (fp32 && A->vfmt == 0 && !A->sval32) return -1.0;
+  if (g_mf_variant < 0 && stencil_ok(A)) return stencil_step_us(A, fp32, B);
   const int Bp = group_width(std::min(B, kMaxB));
   if (autotune(A, fp32, Bp)) return -1.0;
   return (double)A->mf_cost_us[fp32 ? 1 : 0][log2_width(Bp)];
@@ -1122,6 +1162,9 @@ void evslcu_filter_plan_destroy(evslcu_filter_plan *P) {
   if (P->exec) cudaGraphExecDestroy(P->exec);
   evslcu_free(P->work);
   evslcu_free(P->coef);
+  evslcu_free(P->st_mu);
+  free(P->st_cols);
+  free(P->st_off);
   free(P->tab_host);
   delete P;
 }

@@ -1332,6 +1332,7 @@ int evslcu_mat_cheb_grid(const evslcu_mat *A) { return A ? A->cheb_grid : 0; }
 
 double evslcu_chebav_step_cost(evslcu_mat *A) {
   if (!A || A->kernel != 0) return -1.0;
+  if (stencil_ok(A) && g_cheb_force < 0) return stencil_step_us(A, 0, 1);
   const int v = cheb_variant(A);  // tunes on first use
   if (v < 0) return -1.0;
   return A->cheb_best_us > 0.0f ? (double)A->cheb_best_us : (double)A->cheb_us[v];
@@ -1638,10 +1639,36 @@ int evslcu_set_kpm_split(int mode) {
 // KPM dots through the product identities: K = ceil(Mdeg/2) block steps,
 // raw sums a_k = <w_k+1, w_k+1>, b_k = <w_k+1, w_k>, c = <w_0, w_0>; then
 // mu_2k+1 = 2 b_k - mu_1 (mu_1 = b_0) and mu_2k+2 = 2 a_k - c, per probe.
+// dots[(j-1)*B + p] = mu_j, j = 1..Mdeg, from the raw sums [step][sum][probe].
+static void kpm_moments(int Mdeg, int B, const double *raw, double *dots) {
+  const int K = (Mdeg + 1) / 2;
+  for (int p = 0; p < B; ++p) {
+    const double cc0 = raw[2 * (size_t)B + p];  // <w_0, w_0>
+    const double mu1 = raw[(size_t)B + p];      // <w_1, w_0>
+    for (int k = 0; k < K; ++k) {
+      const double a = raw[(size_t)k * 3 * B + p], b = raw[(size_t)k * 3 * B + B + p];
+      const int j1 = 2 * k + 1, j2 = 2 * k + 2;
+      dots[(size_t)(j1 - 1) * B + p] = (k == 0) ? mu1 : 2.0 * b - mu1;
+      if (j2 <= Mdeg) dots[(size_t)(j2 - 1) * B + p] = 2.0 * a - cc0;
+    }
+  }
+}
+
 static int kpm_dots_doubling(const evslcu_op *op, int n, int Mdeg, int nvec, const double *probes, double ctr,
                              double wid, double *dots) {
   const int B = nvec;
   const int K = (Mdeg + 1) / 2;
+  if (stencil_ok(op->A)) {
+    const size_t count = (size_t)K * 3 * B;
+    double *raw = (double *)evslcu_malloc(sizeof(double) * count);
+    if (!raw) return fail(EVSLCU_ERR_NOMEM, "kpm: out of device memory");
+    std::vector<double> hraw(count);
+    int rc = stencil_kpm(op->A, K, B, probes, ctr, wid, raw);
+    if (!rc) rc = evslcu_d2h(hraw.data(), raw, sizeof(double) * count);
+    evslcu_free(raw);
+    if (!rc) kpm_moments(Mdeg, B, hraw.data(), dots);
+    return rc;
+  }
   const size_t blk = (size_t)n * B;
   const int grid = kpm_grid(n);  // a function of n only: the summation order does not depend on B
   // one cached workspace (grows, never shrinks): repeated DOS estimates do
@@ -1714,19 +1741,7 @@ static int kpm_dots_doubling(const evslcu_op *op, int n, int Mdeg, int nvec, con
     }
   }
   if (!rc) rc = evslcu_d2h(hraw.data(), raw, sizeof(double) * hraw.size());
-  if (!rc) {
-    // dots[(j-1)*B + p] = mu_j, j = 1..Mdeg
-    for (int p = 0; p < B; ++p) {
-      const double cc0 = hraw[2 * (size_t)B + p];  // <w_0, w_0>
-      const double mu1 = hraw[(size_t)B + p];      // <w_1, w_0>
-      for (int k = 0; k < K; ++k) {
-        const double a = hraw[(size_t)k * 3 * B + p], b = hraw[(size_t)k * 3 * B + B + p];
-        const int j1 = 2 * k + 1, j2 = 2 * k + 2;
-        dots[(size_t)(j1 - 1) * B + p] = (k == 0) ? mu1 : 2.0 * b - mu1;
-        if (j2 <= Mdeg) dots[(size_t)(j2 - 1) * B + p] = 2.0 * a - cc0;
-      }
-    }
-  }
+  if (!rc) kpm_moments(Mdeg, B, hraw.data(), dots);
   return rc;
 }
 

@@ -107,6 +107,7 @@ struct evslcu_mat {
   void *xs_acc = nullptr;         // partial-sum block of the column-split filter (n x 16 doubles)
   int xs_bad = 0;                 // 1: no column-split copy (a row's columns are not increasing)
   int cheb_ran = 0;           // 1: the single-vector filter has run on the merged stencil
+  unsigned char mf_ran[2][5] = {};  // the same for the multi-column filter, per (fp32, log2 B)
   int cheb_variant = -1;      // single-vector filter kernel chosen by timing (-1: not yet)
   float cheb_us[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // measured time per degree step of each variant
   int cheb_grid = 0;                      // tuned block limit per degree step (0: one row per thread)
@@ -488,6 +489,13 @@ int chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, double cc
 int stencil_build(evslcu_mat *M);
 void stencil_free(evslcu_mat *M);
 bool stencil_ok(const evslcu_mat *M);
+bool stencil_columns_ok(const evslcu_mat *A, int ncols, const evslcu_filter_col *cols);
+double *stencil_columns_mu(int ncols, const evslcu_filter_col *cols, size_t *off, int *err);
+int stencil_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, const double *dmu,
+                    const size_t *off, void *work);
+int stencil_kpm(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw);
+double stencil_step_us(const evslcu_mat *A, int fp32, int n);
+int stencil_batch(int ncols, const evslcu_batch_col *cols, unsigned char *done);
 int stencil_spmv(const evslcu_mat *A, const double *X, double *Y, int m);
 int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,
                    double *work, const evslcu_cheb_epi *epi);

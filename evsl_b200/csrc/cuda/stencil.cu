@@ -50,19 +50,22 @@ struct StMarch {
 // What a degree does to y: terms pending since y was last written (0: none
 // now), their coefficients (c2 w_k-2 + c1 w_k-1 + c0 w_k), and whether y
 // starts with the first of them.
+template <class VT>
 struct StY {
   int terms, init;
-  double c2, c1, c0;
+  VT c2, c1, c0;
 };
 
 // J > 1 needs a stencil whose first and last offsets are -S and +S around a
 // diagonal entry in the middle (StArg::center).
-template <int D, int J, bool FIRST, bool EPI>
-__global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
-    k_st_step(const __grid_constant__ StArg<double, D> A, StMarch M, const double *__restrict__ vk, const double *vkm1,
-              double *out, double *y, double t, double ncc, StY Y, const double *__restrict__ zold, double nbeta,
-              const double *__restrict__ dotv, double *part, unsigned int *ctr, double *dot_out) {
-  __shared__ double sh[EPI ? kThreads / 32 : 1];
+// Returns the sum of dotv[r] y[r] over the thread's rows (EPI).  yd: where the
+// finished y goes (the last degree), else null.
+// each(x, w) is called for every row, with its values of v_k and of the result.
+template <class VT, int D, int J, bool FIRST, bool EPI, class F>
+__device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &M, const VT *__restrict__ vk,
+                                          const VT *vkm1, VT *out, VT *y, double *yd, VT t, VT ncc, const StY<VT> &Y,
+                                          const double *__restrict__ zold, double nbeta,
+                                          const double *__restrict__ dotv, F &&each) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   int r0 = c;
   if (J > 1) {
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
   // has completed once the previous launch has let this one start (it does so
   // after its own wait).
   unsigned m[J];
-  double xm1[J];
+  VT xm1[J];
   bool live[J];
   bool all = true;
 #pragma unroll
@@ -86,22 +89,22 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
     const int r = r0 + j * M.S;
     live[j] = r < A.n;
     m[j] = live[j] ? (unsigned)__ldg(A.mask + r) : 0u;
-    xm1[j] = (!FIRST && live[j]) ? vkm1[r] : 0.0;
+    xm1[j] = (!FIRST && live[j]) ? vkm1[r] : (VT)0;
   }
 #pragma unroll
   for (int j = 0; j < J; ++j) all = all && m[j] == A.full;
   all = __all_sync(0xffffffffu, all);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const double *xr = vk + r0;
-  double acc[J], x[J], yo[J];
+  const VT *xr = vk + r0;
+  VT acc[J], x[J], yo[J];
 #pragma unroll
-  for (int j = 0; j < J; ++j) yo[j] = (Y.terms && !Y.init && live[j]) ? y[r0 + j * M.S] : 0.0;
+  for (int j = 0; j < J; ++j) yo[j] = (Y.terms && !Y.init && live[j]) ? y[r0 + j * M.S] : (VT)0;
   if constexpr (J == 1) {
-    acc[0] = 0.0;
-    x[0] = 0.0;
+    acc[0] = (VT)0;
+    x[0] = (VT)0;
     if (all) {
-      double g[D];
+      VT g[D];
 #pragma unroll
       for (int e = 0; e < D; ++e) g[e] = __ldg(xr + A.off[e]);
 #pragma unroll
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
       x[0] = A.center ? g[D / 2] : __ldg(xr);
     } else {
       // an entry the row does not have adds -0: no change to any sum
-      double g[D];
+      VT g[D];
 #pragma unroll
       for (int e = 0; e < D; ++e) g[e] = (m[0] >> e & 1u) ? __ldg(xr + A.off[e]) : st_zero(A.val[e]);
       if (live[0]) x[0] = __ldg(xr);
@@ -118,7 +121,7 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
     }
   } else {
     // p[j]: the value one S below row j; rows share it with their neighbours
-    double p[J + 2], g[J][D];
+    VT p[J + 2], g[J][D];
     if (all) {
 #pragma unroll
       for (int j = 0; j < J + 2; ++j) p[j] = __ldg(xr + (j - 1) * M.S);
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
           if (e != D / 2) g[j][e] = __ldg(xr + j * M.S + A.off[e]);
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        double a = 0.0;
+        VT a = (VT)0;
 #pragma unroll
         for (int e = 0; e < D; ++e)
           a = st_fmadd(A.val[e], e == 0 ? p[j] : e == D / 2 ? p[j + 1] : e == D - 1 ? p[j + 2] : g[j][e], a);
@@ -139,16 +142,16 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
 #pragma unroll
       for (int j = 0; j < J + 2; ++j) {
         const bool have = j == 0 ? (m[0] & 1u) != 0 : j == J + 1 ? (m[J - 1] >> (D - 1) & 1u) != 0 : live[j == 0 ? 0 : j > J ? J - 1 : j - 1];
-        p[j] = have ? __ldg(xr + (j - 1) * M.S) : 0.0;
+        p[j] = have ? __ldg(xr + (j - 1) * M.S) : (VT)0;
       }
 #pragma unroll
       for (int j = 0; j < J; ++j)
 #pragma unroll
         for (int e = 1; e < D - 1; ++e)
-          if (e != D / 2) g[j][e] = (m[j] >> e & 1u) ? __ldg(xr + j * M.S + A.off[e]) : 0.0;
+          if (e != D / 2) g[j][e] = (m[j] >> e & 1u) ? __ldg(xr + j * M.S + A.off[e]) : (VT)0;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        double a = 0.0;
+        VT a = (VT)0;
 #pragma unroll
         for (int e = 0; e < D; ++e)
           if (m[j] >> e & 1u)
@@ -165,22 +168,39 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
     const int r = r0 + j * M.S;
     if (!live[j]) continue;
     // vkp1 = A vk; vkp1 += (-cc) vk; vkp1 *= t; vkp1 += (-1) vkm1
-    double w = __dmul_rn(t, __dadd_rn(acc[j], __dmul_rn(ncc, x[j])));
-    if (!FIRST) w = __dadd_rn(w, -xm1[j]);
+    VT w = st_mul(t, st_add(acc[j], st_mul(ncc, x[j])));
+    if (!FIRST) w = st_add(w, -xm1[j]);
     out[r] = w;
+    each(x[j], w);
     if (Y.terms) {
-      double yv = yo[j];
-      if (Y.terms == 3) yv = Y.init ? __dmul_rn(Y.c2, xm1[j]) : __dadd_rn(yv, __dmul_rn(Y.c2, xm1[j]));
-      if (Y.terms >= 2)
-        yv = (Y.init && Y.terms == 2) ? __dmul_rn(Y.c1, x[j]) : __dadd_rn(yv, __dmul_rn(Y.c1, x[j]));
-      yv = __dadd_rn(yv, __dmul_rn(Y.c0, w));
-      if (EPI) {
-        if (zold) yv = __dadd_rn(yv, __dmul_rn(nbeta, zold[r]));
-        if (dotv) dsum += dotv[r] * yv;
+      VT yv = yo[j];
+      if (Y.terms == 3) yv = Y.init ? st_mul(Y.c2, xm1[j]) : st_fmadd_y(Y.c2, xm1[j], yv);
+      if (Y.terms >= 2) yv = (Y.init && Y.terms == 2) ? st_mul(Y.c1, x[j]) : st_fmadd_y(Y.c1, x[j], yv);
+      yv = st_fmadd_y(Y.c0, w, yv);
+      if (yd) {
+        double yo2 = (double)yv;
+        if (EPI) {
+          if (zold) yo2 = __dadd_rn(yo2, __dmul_rn(nbeta, zold[r]));
+          if (dotv) dsum += dotv[r] * yo2;
+        }
+        yd[r] = yo2;
+      } else {
+        y[r] = yv;
       }
-      y[r] = yv;
     }
   }
+  return dsum;
+}
+
+template <int D, int J, bool FIRST, bool EPI>
+__global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
+    k_st_step(const __grid_constant__ StArg<double, D> A, StMarch M, const double *__restrict__ vk, const double *vkm1,
+              double *out, double *y, double *yd, double t, double ncc, StY<double> Y,
+              const double *__restrict__ zold, double nbeta, const double *__restrict__ dotv, double *part,
+              unsigned int *ctr, double *dot_out) {
+  __shared__ double sh[EPI ? kThreads / 32 : 1];
+  const double dsum = st_rows<double, D, J, FIRST, EPI>(A, M, vk, vkm1, out, y, yd, t, ncc, Y, zold, nbeta, dotv,
+                                                        [](double, double) {});
   if (EPI && dot_out) {
     const double b = block_sum(dsum, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = b;
@@ -189,6 +209,109 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
       if (threadIdx.x == 0) *dot_out = tot;
     }
   }
+}
+
+// The same degree for several columns of one operator (column in blockIdx.y),
+// each with its own polynomial.  Columns stay apart in memory: the operator
+// costs a byte per row, so there is nothing to share between them, and the
+// vectors of a few columns fit L2 where one interleaved block would not.
+constexpr int kStCols = 16;
+
+template <class VT>
+struct StStepCol {
+  const VT *vk, *vkm1;
+  VT *out, *y;
+  double *yd;        // last degree: where the finished y goes
+  const double *mu;  // device
+  VT t, ncc;
+  int from, flush;  // flush: y takes the terms from .. k now
+};
+template <class VT>
+struct StStepCols {
+  StStepCol<VT> c[kStCols];
+};
+
+template <class VT, int D, int J, bool FIRST>
+__global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
+    k_st_cols(const __grid_constant__ StArg<VT, D> A, StMarch M, const __grid_constant__ StStepCols<VT> C, int k) {
+  const StStepCol<VT> &I = C.c[blockIdx.y];
+  StY<VT> Y{0, 0, (VT)0, (VT)0, (VT)0};
+  if (I.flush) {
+    Y.terms = k - I.from + 1;
+    Y.init = I.from == 0;
+    Y.c0 = (VT)__ldg(I.mu + k);
+    Y.c1 = (VT)__ldg(I.mu + k - 1);
+    Y.c2 = (VT)__ldg(I.mu + (FIRST ? 0 : k - 2));
+  }
+  st_rows<VT, D, J, FIRST, false>(A, M, I.vk, I.vkm1, I.out, I.y, I.yd, I.t, I.ncc, Y, nullptr, 0.0, nullptr,
+                                  [](VT, VT) {});
+}
+
+// One KPM step (two moments per product, as k_kpm_dbl in sparse.cu) for the
+// probes of a group, probe in blockIdx.y, vectors of n values one after
+// another: w_k+1 and the block's sums of w_k+1^2, w_k+1 w_k and, at the first
+// step, w_0^2, into part[(sum * probes + probe) * blocks + block].  The blocks,
+// and so the order of the sums, follow from n alone.
+template <int D, int J, bool FIRST>
+__global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
+    k_st_kpm(const __grid_constant__ StArg<double, D> A, StMarch M, const double *__restrict__ vk, const double *vkm1,
+             double *out, double t, double ncc, double *part) {
+  __shared__ double sh[kThreads / 32];
+  const long long at = (long long)blockIdx.y * A.n;
+  double s[3] = {0.0, 0.0, 0.0};
+  const StY<double> Y{0, 0, 0.0, 0.0, 0.0};
+  st_rows<double, D, J, FIRST, false>(A, M, vk + at, FIRST ? nullptr : vkm1 + at, out + at, nullptr, nullptr, t, ncc,
+                                      Y, nullptr, 0.0, nullptr, [&](double x, double w) {
+                                        s[0] += w * w;
+                                        s[1] += w * x;
+                                        if (FIRST) s[2] += x * x;
+                                      });
+#pragma unroll
+  for (int q = 0; q < (FIRST ? 3 : 2); ++q) {
+    const double b = block_sum(s[q], sh);
+    if (threadIdx.x == 0) part[((long long)q * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = b;
+  }
+}
+
+// The sums of several steps, step and sum in blockIdx.y, probe of the group in
+// blockIdx.x: part's `blocks` entries in fixed order.  raw: [step * 3 + sum]
+// [all probes], at this group's first probe.
+__global__ void __launch_bounds__(kThreads)
+    k_st_kpm_sum(int blocks, const double *__restrict__ part, double *raw, int nvec) {
+  __shared__ double sh[kThreads / 32];
+  const double *p = part + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blocks;
+  double t = 0.0;
+  for (int i = threadIdx.x; i < blocks; i += kThreads) t += p[i];
+  t = block_sum(t, sh);
+  if (threadIdx.x == 0) raw[(long long)blockIdx.y * nvec + blockIdx.x] = t;
+}
+
+// Unit probes: block b of a probe's 64 sums its squares, then every block
+// scales its share (two launches; the sums' order follows from n alone).
+constexpr int kNormBlocks = 64;
+__global__ void __launch_bounds__(kThreads) k_st_sumsq(int n, const double *__restrict__ x, double *part) {
+  __shared__ double sh[kThreads / 32];
+  const double *xc = x + (long long)blockIdx.y * n;
+  double t = 0.0;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) t += xc[r] * xc[r];
+  t = block_sum(t, sh);
+  if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+}
+__global__ void __launch_bounds__(kThreads) k_st_unit(int n, const double *__restrict__ x, const double *part, double *v) {
+  __shared__ double inv;
+  if (threadIdx.x < 32) {
+    double t = part[blockIdx.y * kNormBlocks + threadIdx.x] + part[blockIdx.y * kNormBlocks + 32 + threadIdx.x];
+    t = warp_sum(t);
+    if (threadIdx.x == 0) inv = 1.0 / sqrt(t);
+  }
+  __syncthreads();
+  const double s = inv;
+  const long long at = (long long)blockIdx.y * n;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) v[at + r] = __dmul_rn(s, x[at + r]);
+}
+
+__global__ void k_st_float(int n, const double *__restrict__ x, float *out) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) out[r] = (float)x[r];
 }
 
 // Two rows per thread where the grid still covers every SM's warps about
@@ -211,7 +334,7 @@ StMarch st_march(int n, int span, bool sym) {
 
 template <int D>
 int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y, double t,
-            double ncc, const StY &Y, const evslcu_cheb_epi *ep) {
+            double ncc, const StY<double> &Y, bool last, const evslcu_cheb_epi *ep) {
   const StArg<double, D> S = st_arg<double, D>(A);
   const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
   cudaLaunchConfig_t cfg = {};
@@ -230,7 +353,7 @@ int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm
                  : (epi ? k_st_step<D, J, false, true> : k_st_step<D, J, false, false>);
   };
   auto fn = M.J == 2 ? pick(std::integral_constant<int, 2>()) : pick(std::integral_constant<int, 1>());
-  cudaError_t e = cudaLaunchKernelEx(&cfg, fn, S, M, vk, vkm1, out, y, t, ncc, Y,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, fn, S, M, vk, vkm1, out, y, last ? y : nullptr, t, ncc, Y,
                                      epi ? ep->zold : nullptr, epi ? ep->nbeta : 0.0, epi ? ep->dotv : nullptr,
                                      partials(), counters() + CTR_CHEB, epi ? ep->dot_out : nullptr);
   if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "stencil filter launch failed: %s", cudaGetErrorString(e));
@@ -240,13 +363,13 @@ int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm
 }
 
 int st_step_any(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y, double t,
-                double ncc, const StY &Y, const evslcu_cheb_epi *ep) {
+                double ncc, const StY<double> &Y, bool last, const evslcu_cheb_epi *ep) {
   switch (st_width(A->st_d)) {
-    case 5: return st_step<5>(A, first, vk, vkm1, out, y, t, ncc, Y, ep);
-    case 7: return st_step<7>(A, first, vk, vkm1, out, y, t, ncc, Y, ep);
-    case 9: return st_step<9>(A, first, vk, vkm1, out, y, t, ncc, Y, ep);
-    case 16: return st_step<16>(A, first, vk, vkm1, out, y, t, ncc, Y, ep);
-    default: return st_step<32>(A, first, vk, vkm1, out, y, t, ncc, Y, ep);
+    case 5: return st_step<5>(A, first, vk, vkm1, out, y, t, ncc, Y, last, ep);
+    case 7: return st_step<7>(A, first, vk, vkm1, out, y, t, ncc, Y, last, ep);
+    case 9: return st_step<9>(A, first, vk, vkm1, out, y, t, ncc, Y, last, ep);
+    case 16: return st_step<16>(A, first, vk, vkm1, out, y, t, ncc, Y, last, ep);
+    default: return st_step<32>(A, first, vk, vkm1, out, y, t, ncc, Y, last, ep);
   }
 }
 
@@ -384,12 +507,15 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
 // later waits of the block give up at once, and it stays until the blocks that
 // may still send to it are done.
 //
+// MANY: the launch's blocks may have more threads than this column's rows need
+// (R is a multiple of a warp, so whole warps sit out).
+//
 // ONE: at most one row per thread, whose w_k, w_k-1 and y stay in registers.
 // The instruction count per row is what bounds a degree (a first version with
 // its first / last / y tests inside the row loop took 130-190 instructions per
 // 32 rows: 0.97 us a degree on 10^4 rows, 3.8 us on 94,800), so those cases
 // are compiled apart.
-template <class VT, int D, bool ONE, class MU>
+template <class VT, int D, bool ONE, bool MANY, class MU>
 __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls, int *err) {
   constexpr int VB = (int)sizeof(VT);
   extern __shared__ __align__(16) unsigned char st_smem[];
@@ -422,10 +548,11 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
   }
   // R = nit T rows, those past n empty ones; the last T are visited first, so
   // that the rows both neighbours wait for come early.
-  const int nit = ONE ? 1 : R / T;
+  const int nit = ONE ? 1 : (R + T - 1) / T;
   // bit `it`: the warp's rows of iteration `it` have every entry / read a halo
   unsigned fast = 0, edge = 0, m1 = 0;
   for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T) {
+    if (MANY && i >= R) continue;
     m1 = i < rows ? (unsigned)__ldg(mask + i) : 0u;
     if (!ONE) ms[i] = (MT)m1;
     if (__all_sync(0xffffffffu, m1 == I.full)) fast |= 1u << it;
@@ -476,6 +603,7 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
     unsigned fb = fast, eb = edge;
 #pragma unroll 2
     for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T, fb >>= 1, eb >>= 1) {
+      if (MANY && i >= R) continue;
       const VT *xs = src + i;
       VT acc = (VT)0, x, xm1 = (VT)0;
       if (!FIRST) xm1 = ONE ? rm : dst[i];
@@ -589,23 +717,199 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
   }
 }
 
-// CAP >= 0: one cluster filters `one`, whose coefficients (up to CAP) come
-// with the launch, or from the device when CAP is 0.  CAP -1: cluster q of
-// the launch filters tab[q].
+// One cluster filters `one`, whose coefficients (up to CAP) come with the
+// launch, or from the device when CAP is 0.
 template <class VT, int D, int CAP, bool ONE>
 __global__ void __launch_bounds__(cl_threads(CAP, ONE), 1)
-    k_st_cluster(const StCol *__restrict__ tab, const __grid_constant__ StCol one,
-                 const __grid_constant__ StMu<CAP> mus, int polls, int *err) {
+    k_st_cluster(const __grid_constant__ StCol one, const __grid_constant__ StMu<CAP> mus, int polls, int *err) {
   if constexpr (CAP > 0) {
-    st_cluster_body<VT, D, ONE>(one, [&](int k) { return mus.v[k]; }, polls, err);
-  } else if constexpr (CAP == 0) {
-    const double *mup = one.mu;
-    st_cluster_body<VT, D, ONE>(one, [&](int k) { return __ldg(mup + k); }, polls, err);
+    st_cluster_body<VT, D, ONE, false>(one, [&](int k) { return mus.v[k]; }, polls, err);
   } else {
-    const StCol &I = tab[blockIdx.x / cluster_size()];
-    const double *mup = I.mu;
-    st_cluster_body<VT, D, ONE>(I, [&](int k) { return __ldg(mup + k); }, polls, err);
+    const double *mup = one.mu;
+    st_cluster_body<VT, D, ONE, false>(one, [&](int k) { return __ldg(mup + k); }, polls, err);
   }
+}
+
+// Cluster q of the launch filters column q of the table, whatever its
+// operator: columns of one matrix, or of as many matrices.
+constexpr int kClCols = 32;
+struct StTab {
+  StCol c[kClCols];
+};
+template <class VT, int D, bool ONE>
+__global__ void __launch_bounds__(cl_threads(-1, ONE), 1)
+    k_st_clusters(const __grid_constant__ StTab tab, int polls, int *err) {
+  const StCol &I = tab.c[blockIdx.x / cluster_size()];
+  const double *mup = I.mu;
+  st_cluster_body<VT, D, ONE, true>(I, [&](int k) { return __ldg(mup + k); }, polls, err);
+}
+
+// The whole KPM recurrence of a probe (k_st_kpm's steps, the probe made a unit
+// vector first) on one cluster: cluster q of the launch takes probe q of x.
+// Vectors, halos and waits are st_cluster_body's.  Block c of probe q leaves
+// its sums of step k in part[((k * 3 + sum) * probes + q) * blocks + c].
+template <int D, bool ONE>
+__global__ void __launch_bounds__(cl_threads(0, ONE), 1)
+    k_st_kpm_cluster(const __grid_constant__ StCol I, double *part, int probes, int polls, int *err) {
+  constexpr int VB = (int)sizeof(double);
+  extern __shared__ __align__(16) unsigned char st_smem[];
+  __shared__ double red[64];
+  __shared__ double sums[2][3][32];
+  __shared__ __align__(16) unsigned long long bars[2];
+  __shared__ int dead;
+  double *const sm = reinterpret_cast<double *>(st_smem);
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+  const int cr = (int)cluster_rank(), cl = (int)cluster_size(), probe = (int)(blockIdx.x / cl);
+  const int R = I.R, H = I.halo, n = I.n, steps = I.deg;
+  const int row0 = cr * R;
+  const int rows = max(0, min(R, n - row0));
+  using MT = typename StMaskT<D>::T;
+  const MT *const mask = (const MT *)I.mask + row0;
+  const double *const x0 = I.x + (long long)probe * n;
+  const bool low = cr > 0 && rows > 0, high = cr + 1 < cl && row0 + R < n;
+  double *src = sm + H, *dst = sm + (R + 2 * H) + H;
+  MT *const ms = reinterpret_cast<MT *>(sm + 2 * (R + 2 * H));
+  if (tid == 0) {
+    bar_init(bars);
+    bar_init(bars + 1);
+    dead = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  double sq = 0.0;
+  for (int i = tid - H; i < R + H; i += T) {
+    const int g = row0 + i;
+    if (g >= 0 && g < n) {
+      const double v = x0[g];
+      src[i] = v;
+      if (i >= 0 && i < R) sq += v * v;
+    }
+  }
+  const int nit = ONE ? 1 : R / T;
+  unsigned fast = 0, edge = 0, m1 = 0;
+  for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T) {
+    m1 = i < rows ? (unsigned)__ldg(mask + i) : 0u;
+    if (!ONE) ms[i] = (MT)m1;
+    if (__all_sync(0xffffffffu, m1 == I.full)) fast |= 1u << it;
+    if (__any_sync(0xffffffffu, i < rows && ((low && i < H) || (high && i >= R - H)))) edge |= 1u << it;
+  }
+  // the probe's norm: every block's sum in every block, added in rank order
+  sq = block_sum(sq, red);
+  if (cl > 1) {
+    cluster_sync();
+    if (tid == 0)
+      for (int c = 0; c < cl; ++c) peer_store(peer_addr(red + 32 + cr, c), sq);
+    cluster_sync();
+  } else {
+    if (tid == 0) red[32] = sq;
+    __syncthreads();
+  }
+  double tot = 0.0;
+  for (int c = 0; c < cl; ++c) tot += red[32 + c];
+  const double inv = 1.0 / sqrt(tot);
+  for (int i = tid - H; i < R + H; i += T) {
+    const int g = row0 + i;
+    if (g >= 0 && g < n) src[i] = __dmul_rn(inv, src[i]);
+  }
+  __syncthreads();
+  unsigned dl = low ? peer_addr(dst, cr - 1) + R * VB : 0, sl = low ? peer_addr(src, cr - 1) + R * VB : 0;
+  unsigned dh = high ? peer_addr(dst, cr + 1) - R * VB : 0, sh = high ? peer_addr(src, cr + 1) - R * VB : 0;
+  const unsigned bl = low ? peer_addr(bars, cr - 1) : 0, bh = high ? peer_addr(bars, cr + 1) : 0;
+  const unsigned expect = (low ? (unsigned)(H * VB) : 0u) + (high ? (unsigned)(min(H, n - row0 - R) * VB) : 0u);
+  const bool center = I.center != 0;
+  double rx = (ONE && tid < rows) ? src[tid] : 0.0, rm = 0.0;
+  // a neighbour's first rows may arrive only after it has read its own probe,
+  // and go to the other vector: no barrier is needed before the first step
+  auto step = [&](int k, auto first_c) {  // k = 1, 2, ... as a filter's degrees
+    constexpr bool FIRST = decltype(first_c)::value;
+    const bool last = k == steps;
+    const double t = FIRST ? I.t1 : I.t2;
+    if (!last && tid == 0 && expect && !*(volatile int *)&dead) bar_expect(bars + (k & 1), expect);
+    if (!FIRST && edge && !bar_wait(bars + ((k - 1) & 1), (unsigned)((k - 2) >> 1) & 1u, polls, &dead)) {
+      *(volatile int *)&dead = 1;
+      *(volatile int *)err = 1;
+    }
+    const unsigned bk = (unsigned)((k & 1) * 8);
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    unsigned fb = fast, eb = edge;
+    for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T, fb >>= 1, eb >>= 1) {
+      const double *xs = src + i;
+      double acc = 0.0, x, xm1 = 0.0, g[D];
+      if (!FIRST) xm1 = ONE ? rm : dst[i];
+      if (fb & 1u) {
+#pragma unroll
+        for (int e = 0; e < D; ++e)
+          if (!ONE || e != D / 2) g[e] = xs[I.off[e]];
+        if (ONE) g[D / 2] = center ? rx : xs[I.off[D / 2]];
+        x = ONE ? rx : center ? g[D / 2] : xs[0];
+      } else {
+        const unsigned m = ONE ? m1 : (unsigned)ms[i];
+#pragma unroll
+        for (int e = 0; e < D; ++e) {
+          g[e] = st_zero(I.val[e]);
+          if (m >> e & 1u) g[e] = xs[I.off[e]];
+        }
+        x = ONE ? rx : xs[0];
+      }
+#pragma unroll
+      for (int e = 0; e < D; ++e) acc = st_fmadd(I.val[e], g[e], acc);
+      double w = __dmul_rn(t, __dadd_rn(acc, __dmul_rn(I.ncc, x)));
+      if (!FIRST) w = __dadd_rn(w, -xm1);
+      if (!last) {
+        if ((eb & 1u) && i < rows) {
+          if (low && i < H) peer_send(dl + (unsigned)(i * VB), w, bl + bk);
+          if (high && i >= R - H) peer_send(dh + (unsigned)(i * VB), w, bh + bk);
+        }
+        dst[i] = w;
+      }
+      if (i < rows) {
+        s0 += w * w;
+        s1 += w * x;
+        if (FIRST) s2 += x * x;
+      }
+      if (ONE) {
+        rm = rx;
+        rx = w;
+      }
+    }
+    // the step's sums: one per warp now, the block's by warp 0 after the barrier
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
+    if (FIRST) s2 = warp_sum(s2);
+    if (lane == 0) {
+      sums[k & 1][0][warp] = s0;
+      sums[k & 1][1][warp] = s1;
+      if (FIRST) sums[k & 1][2][warp] = s2;
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int q = 0; q < (FIRST ? 3 : 2); ++q) {
+        const double b = warp_sum(lane < nw ? sums[k & 1][q][lane] : 0.0);
+        if (lane == 0) part[((long long)((k - 1) * 3 + q) * probes + probe) * cl + cr] = b;
+      }
+    }
+    double *const pv = src;
+    src = dst;
+    dst = pv;
+    unsigned q = sl;
+    sl = dl;
+    dl = q;
+    q = sh;
+    sh = dh;
+    dh = q;
+  };
+  step(1, std::true_type{});
+  for (int k = 2; k <= steps; ++k) step(k, std::false_type{});
+  if (cl > 1 && dead) cluster_sync();  // nobody's memory goes away while others may still send to it
+}
+
+// raw[i] = part[i * cl] + part[i * cl + 1] + ...
+__global__ void k_st_kpm_cl_sum(int count, int cl, const double *__restrict__ part, double *raw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  double s = 0.0;
+  for (int c = 0; c < cl; ++c) s += part[(long long)i * cl + c];
+  raw[i] = s;
 }
 
 // Blocks of the cluster, rows and shared memory of one column; cl 0: none fits.
@@ -651,22 +955,17 @@ ClPlan cl_plan(int n, int reach, int d, size_t vb, int cl, int cap) {
 int g_cl_force = 0;  // blocks per cluster: 0 the rule below, -1 no cluster
 
 // Most blocks per cluster this device runs (16 is above the portable 8).
-template <class VT, int D, int CAP, bool ONE>
-int cl_max1() {
-  static int m = 0;
-  if (m) return m;
-  const void *fn = (const void *)k_st_cluster<VT, D, CAP, ONE>;
-  m = -1;
+int cl_limit(const void *fn, int threads) {
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax) != cudaSuccess) {
     cudaGetLastError();
-    return m;
+    return -1;
   }
   const bool wide = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
   if (!wide) cudaGetLastError();
   for (int cl = wide ? 16 : 8; cl >= 1; cl /= 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(cl_threads(CAP, ONE));
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = kClSmemMax;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -675,13 +974,10 @@ int cl_max1() {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int got = 0;
-    if (cudaOccupancyMaxActiveClusters(&got, fn, &cfg) == cudaSuccess && got >= 1) {
-      m = cl;
-      break;
-    }
+    if (cudaOccupancyMaxActiveClusters(&got, fn, &cfg) == cudaSuccess && got >= 1) return cl;
     cudaGetLastError();
   }
-  return m;
+  return -1;
 }
 
 int *g_cl_err = nullptr;  // mapped host flag: a wait of the cluster filter ran out
@@ -699,19 +995,30 @@ int *cl_err() {
   return g_cl_err;
 }
 
+template <class VT, int D, int CAP, bool ONE>
+int cl_max1() {
+  static int m = 0;
+  if (m) return m;
+  if constexpr (CAP < 0)
+    m = cl_limit((const void *)k_st_clusters<VT, D, ONE>, cl_threads(CAP, ONE));
+  else
+    m = cl_limit((const void *)k_st_cluster<VT, D, CAP, ONE>, cl_threads(CAP, ONE));
+  return m;
+}
+
 template <class VT, int D, int CAP>
 int cl_max() {
   return std::min(cl_max1<VT, D, CAP, true>(), cl_max1<VT, D, CAP, false>());
 }
 
 template <class VT, int D, int CAP>
-int cl_launch(int ncols, const StCol *tab, const StCol &one, const double *mu, const ClPlan &P) {
+int cl_launch(const StCol &one, const double *mu, const ClPlan &P) {
   int *err = cl_err();  // same address on the device (unified addressing)
   if (!err) return fail(EVSLCU_ERR_NOMEM, "cluster filter: out of pinned host memory");
   StMu<CAP> mus;
   if (CAP > 0) memcpy(mus.v, mu, sizeof(double) * (size_t)(one.deg + 1));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(P.cl * ncols);
+  cfg.gridDim = dim3(P.cl);
   cfg.blockDim = dim3(P.T);
   cfg.dynamicSmemBytes = P.smem;
   cfg.stream = stream();
@@ -721,8 +1028,8 @@ int cl_launch(int ncols, const StCol *tab, const StCol &one, const double *mu, c
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, true>, tab, one, mus, kClPolls, err)
-                           : cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, false>, tab, one, mus, kClPolls, err);
+  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, true>, one, mus, kClPolls, err)
+                           : cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, false>, one, mus, kClPolls, err);
   if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "cluster filter launch failed: %s", cudaGetErrorString(e));
   EVSLCU_LAUNCH_CHECK("k_st_cluster");
   return 0;
@@ -732,16 +1039,37 @@ template <class VT, int CAP>
 int cl_most(int d) {
   return d <= 5 ? cl_max<VT, 5, CAP>() : d <= 7 ? cl_max<VT, 7, CAP>() : cl_max<VT, 9, CAP>();
 }
-// `one`: the column, or for a table its widest stencil.
 template <class VT, int CAP>
-int cl_launch_d(int ncols, const StCol *tab, const StCol &one, const double *mu, const ClPlan &P) {
-  return one.d <= 5   ? cl_launch<VT, 5, CAP>(ncols, tab, one, mu, P)
-         : one.d <= 7 ? cl_launch<VT, 7, CAP>(ncols, tab, one, mu, P)
-                      : cl_launch<VT, 9, CAP>(ncols, tab, one, mu, P);
+int cl_launch_d(const StCol &one, const double *mu, const ClPlan &P) {
+  return one.d <= 5   ? cl_launch<VT, 5, CAP>(one, mu, P)
+         : one.d <= 7 ? cl_launch<VT, 7, CAP>(one, mu, P)
+                      : cl_launch<VT, 9, CAP>(one, mu, P);
+}
+
+template <class VT, int D>
+int cl_launch_many(int ncols, const StTab &tab, int cl, int T, size_t smem, bool one) {
+  int *err = cl_err();
+  if (!err) return fail(EVSLCU_ERR_NOMEM, "cluster filter: out of pinned host memory");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl * ncols);
+  cfg.blockDim = dim3(T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = one ? cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, true>, tab, kClPolls, err)
+                      : cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, false>, tab, kClPolls, err);
+  if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "cluster filter launch failed: %s", cudaGetErrorString(e));
+  EVSLCU_LAUNCH_CHECK("k_st_clusters");
+  return 0;
 }
 
 void cl_column(StCol &C, const evslcu_mat *A, int deg, double cc, double dd, const double *x, double *y,
-               const ClPlan &P) {
+               const ClPlan &P, int D) {
   memset(&C, 0, sizeof(C));
   C.mask = A->st_mask;
   C.x = x;
@@ -755,7 +1083,7 @@ void cl_column(StCol &C, const evslcu_mat *A, int deg, double cc, double dd, con
   C.R = P.R;
   C.halo = P.halo;
   C.y_smem = P.y_smem;
-  const int D = st_width(A->st_d);
+  // D: the compiled width (of the launch's widest stencil)
   C.full = A->st_d == D ? (1u << D) - 1u : 0xffffffffu;
   C.center = A->st_d == D && A->st_off[D / 2] == 0;
   for (int e = 0; e < A->st_d; ++e) {
@@ -786,7 +1114,7 @@ int cl_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double 
     P = cl_plan(A->n, A->st_reach, A->st_d, sizeof(double), std::min(cl, most), 0);
   if (!P.cl || (!g_cl_force && P.R > (A->st_d <= 5 ? kClMostRows5 : kClMostRows9))) return 0;
   StCol C;
-  cl_column(C, A, deg, cc, dd, v, y, P);
+  cl_column(C, A, deg, cc, dd, v, y, P, st_width(A->st_d));
   if (epi) {
     C.zold = epi->zold;
     C.nbeta = epi->nbeta;
@@ -794,8 +1122,8 @@ int cl_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double 
     C.dot_out = epi->dot_out;
   }
   *done = true;
-  if (deg < 64) return cl_launch_d<double, 64>(1, nullptr, C, mu, P);
-  if (deg < 512) return cl_launch_d<double, 512>(1, nullptr, C, mu, P);
+  if (deg < 64) return cl_launch_d<double, 64>(C, mu, P);
+  if (deg < 512) return cl_launch_d<double, 512>(C, mu, P);
   if (deg + 1 > g_cl_mu_cap) {
     evslcu_free(g_cl_mu);
     g_cl_mu_cap = std::max(deg + 1, 4096);
@@ -808,7 +1136,300 @@ int cl_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double 
   const int rc = evslcu_h2d_async(g_cl_mu, mu, sizeof(double) * (size_t)(deg + 1));
   if (rc) return rc;
   C.mu = g_cl_mu;
-  return cl_launch_d<double, 0>(1, nullptr, C, nullptr, P);
+  return cl_launch_d<double, 0>(C, nullptr, P);
+}
+
+// Columns filtered together on clusters: col[i] of operator A[i], degree >= 1,
+// coefficients on the device.
+struct ClMany {
+  const evslcu_mat *A;
+  const double *mu;
+  int deg;
+  double cc, dd;
+  const double *x;
+  double *y;
+};
+
+// Most blocks per cluster of those launches.
+int cl_many_most(size_t vb) {
+  if (vb == sizeof(float)) return std::min(cl_most<float, -1>(5), std::min(cl_most<float, -1>(7), cl_most<float, -1>(9)));
+  return std::min(cl_most<double, -1>(5), std::min(cl_most<double, -1>(7), cl_most<double, -1>(9)));
+}
+
+// Plan of one column in a launch of cl blocks per column and precision vb.
+ClPlan cl_plan_many(const evslcu_mat *A, size_t vb, int cl) {
+  if (A->st_d > kClMaxD) return ClPlan();
+  return cl_plan(A->n, A->st_reach, A->st_d, vb, cl, -1);
+}
+
+// Filters n columns (each of which has a plan) in launches of up to kClCols
+// clusters; a launch's operators have masks of one type.  It takes the largest
+// cluster that still lets its columns run at once.
+template <class VT>
+int cl_many(int n, const ClMany *cols) {
+  const int most = cl_many_most(sizeof(VT));
+  for (int c0 = 0, nc; c0 < n; c0 += nc) {
+    nc = 1;
+    const int mb = st_mask_bytes(cols[c0].A->st_d);
+    while (nc < kClCols && c0 + nc < n && st_mask_bytes(cols[c0 + nc].A->st_d) == mb) ++nc;
+    // the smallest cluster every column fits, then larger while they all run at once
+    int cl = 0;
+    for (int t = 1; t <= most; t *= 2) {
+      bool fits = true;
+      for (int i = 0; i < nc && fits; ++i) fits = cl_plan_many(cols[c0 + i].A, sizeof(VT), t).cl > 0;
+      if (fits && (!cl || t * nc <= sm_count())) cl = t;
+    }
+    if (!cl) return fail(EVSLCU_ERR_ARG, "cluster filter: a column does not fit");
+    StTab tab;
+    int D = 5, T = 0;
+    size_t smem = 0;
+    bool one = true;
+    for (int i = 0; i < nc; ++i) D = std::max(D, st_width(cols[c0 + i].A->st_d));
+    for (int i = 0; i < nc; ++i) {
+      const ClMany &c = cols[c0 + i];
+      const ClPlan P = cl_plan_many(c.A, sizeof(VT), cl);
+      cl_column(tab.c[i], c.A, c.deg, c.cc, c.dd, c.x, c.y, P, D);
+      tab.c[i].mu = c.mu;
+      T = std::max(T, P.T);
+      // (a plan of one row per thread has no room for the masks)
+      smem = std::max(smem, P.smem + (P.R == P.T ? (size_t)P.R * mb : 0));
+      one = one && P.R == P.T;
+    }
+    const int rc = D == 5   ? cl_launch_many<VT, 5>(nc, tab, cl, T, smem, one)
+                   : D == 7 ? cl_launch_many<VT, 7>(nc, tab, cl, T, smem, one)
+                            : cl_launch_many<VT, 9>(nc, tab, cl, T, smem, one);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+// Whether n columns of A go to clusters rather than to one launch per degree:
+// most blocks a column may have, and the time of a degree of all columns on
+// either, as measured: on a cluster 0.45 us plus 0.7 (5-point) or 1.15 us per
+// thousand rows of a block above one row per thread; k_st_cols 2.2 us a launch
+// plus 6.3 (FP32: 3.6) us per million rows.
+bool cl_columns_pay(const evslcu_mat *A, size_t vb, int n, double *us = nullptr) {
+  const double step = 2.2 + (vb == 8 ? 6.3e-6 : 3.6e-6) * (double)A->n * n;
+  if (us) *us = step;
+  if (A->st_d > kClMaxD || g_cl_force < 0) return false;
+  const int most = cl_many_most(vb);
+  int cl = 0;
+  for (int t = 1; t <= most; t *= 2)
+    if (cl_plan_many(A, vb, t).cl && (!cl || t * std::min(n, kClCols) <= sm_count())) cl = t;
+  if (!cl) return false;
+  const ClPlan P = cl_plan_many(A, vb, cl);
+  const double deg1 = 0.45 + (P.R > 512 ? (A->st_d <= 5 ? 0.7e-3 : 1.15e-3) * P.R : 0.0);
+  const double waves = std::max(1.0, std::ceil((double)n * cl / sm_count()));
+  if (us) *us = std::min(step, waves * deg1);
+  return g_cl_force > 0 || waves * deg1 < step;
+}
+
+template <class VT, int D>
+int st_cols_launch(const evslcu_mat *A, int na, const StStepCols<VT> &C, int k) {
+  const StArg<VT, D> S = st_arg<VT, D>(A);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads, na);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  constexpr int J2 = D <= 9 ? 2 : 1;
+  auto fn = M.J == 2 ? (k == 1 ? k_st_cols<VT, D, J2, true> : k_st_cols<VT, D, J2, false>)
+                     : (k == 1 ? k_st_cols<VT, D, 1, true> : k_st_cols<VT, D, 1, false>);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, fn, S, M, C, k);
+  if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "stencil filter launch failed: %s", cudaGetErrorString(e));
+  EVSLCU_LAUNCH_CHECK("k_st_cols");
+  return 0;
+}
+
+// Bytes of recurrence vectors that a group of columns may have at once: they
+// stay in L2 from degree to degree.
+constexpr size_t kStColsBytes = (size_t)80 << 20;
+
+// nc (at most kStCols) columns of A, one launch per degree; work: 4 vectors of
+// n VT per column.
+template <class VT>
+int st_cols_group(const evslcu_mat *A, int nc, const ClMany *cols, VT *work) {
+  const size_t n = (size_t)A->n;
+  int order[kStCols], from[kStCols] = {};
+  for (int i = 0; i < nc; ++i) order[i] = i;
+  std::stable_sort(order, order + nc, [&](int p, int q) { return cols[p].deg > cols[q].deg; });
+  constexpr bool F32 = sizeof(VT) == 4;
+  if constexpr (F32) {
+    for (int i = 0; i < nc; ++i) {
+      k_st_float<<<grid_for(A->n), kThreads, 0, stream()>>>(A->n, cols[i].x, (float *)work + (size_t)(4 * i + 2) * n);
+      EVSLCU_LAUNCH_CHECK("k_st_float");
+    }
+  }
+  int active = nc;
+  StStepCols<VT> C;
+  memset(&C, 0, sizeof(C));
+  for (int k = 1; k <= cols[order[0]].deg; ++k) {
+    while (cols[order[active - 1]].deg < k) --active;
+    for (int a = 0; a < active; ++a) {
+      const int i = order[a];
+      const ClMany &c = cols[i];
+      VT *W[2] = {work + (size_t)(4 * i) * n, work + (size_t)(4 * i + 1) * n};
+      const VT *x0;
+      VT *y;
+      if constexpr (F32) {
+        x0 = work + (size_t)(4 * i + 2) * n;
+        y = work + (size_t)(4 * i + 3) * n;
+      } else {
+        x0 = c.x;
+        y = c.y;
+      }
+      StStepCol<VT> &I = C.c[a];
+      I.vk = (k == 1) ? x0 : W[(k - 2) % 2];
+      I.vkm1 = (k == 1) ? nullptr : ((k == 2) ? x0 : W[(k - 1) % 2]);
+      I.out = W[(k - 1) % 2];
+      I.y = y;
+      I.yd = k == c.deg ? c.y : nullptr;
+      I.mu = c.mu;
+      I.t = (VT)((k == 1) ? 1.0 / c.dd : 2.0 / c.dd);
+      I.ncc = (VT)(-c.cc);
+      I.from = from[i];
+      I.flush = k == c.deg || k - from[i] == 2;
+      if (I.flush) from[i] = k + 1;
+    }
+    int rc;
+    switch (st_width(A->st_d)) {
+      case 5: rc = st_cols_launch<VT, 5>(A, active, C, k); break;
+      case 7: rc = st_cols_launch<VT, 7>(A, active, C, k); break;
+      case 9: rc = st_cols_launch<VT, 9>(A, active, C, k); break;
+      case 16: rc = st_cols_launch<VT, 16>(A, active, C, k); break;
+      default: rc = st_cols_launch<VT, 32>(A, active, C, k); break;
+    }
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+// The KPM recurrence of nvec probes on clusters; *done stays false when the
+// operator is too large.  The plan follows from n alone, so that a probe's sums
+// do not depend on the others.
+template <int D>
+int kpm_cluster(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw,
+                bool *done) {
+  static int most = 0;  // most blocks per cluster, as cl_max1
+  const void *fn1 = (const void *)k_st_kpm_cluster<D, true>, *fn2 = (const void *)k_st_kpm_cluster<D, false>;
+  if (!most) {
+    most = std::min(cl_limit(fn1, cl_threads(0, true)), cl_limit(fn2, cl_threads(0, false)));
+  }
+  ClPlan P;
+  for (int cl = 1; cl <= most; cl *= 2) {
+    const ClPlan Q = cl_plan(A->n, A->st_reach, A->st_d, sizeof(double), cl, 0);
+    if (Q.cl) P = Q;
+    if (Q.cl && Q.R == Q.T) break;  // the smallest cluster with one row per thread, else the largest
+  }
+  if (!P.cl || (g_cl_force == 0 && P.R > (A->st_d <= 5 ? kClMostRows5 : kClMostRows9))) return 0;
+  int *err = cl_err();
+  if (!err) return fail(EVSLCU_ERR_NOMEM, "KPM: out of pinned host memory");
+  StCol C;
+  cl_column(C, A, steps, ctr, wid, probes, nullptr, P, st_width(A->st_d));
+  const size_t count = (size_t)steps * 3 * nvec;
+  double *part = (double *)evslcu_malloc(sizeof(double) * count * P.cl);
+  if (!part) return EVSLCU_ERR_NOMEM;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(P.cl * nvec);
+  cfg.blockDim = dim3(P.T);
+  cfg.dynamicSmemBytes = P.smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = P.cl;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, true>, C, part, nvec, kClPolls, err)
+                             : cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, false>, C, part, nvec, kClPolls, err);
+  int rc = e == cudaSuccess ? 0 : fail(EVSLCU_ERR_CUDA, "KPM cluster launch failed: %s", cudaGetErrorString(e));
+  count_launch();
+  if (!rc) rc = check_launch("k_st_kpm_cluster");
+  if (!rc) {
+    // (the third sum exists at the first step only; its other places are not read)
+    k_st_kpm_cl_sum<<<grid_for((long long)count), kThreads, 0, stream()>>>((int)count, P.cl, part, raw);
+    count_launch();
+    rc = check_launch("k_st_kpm_cl_sum");
+  }
+  evslcu_free(part);
+  *done = true;
+  return rc;
+}
+
+template <int D>
+int kpm_steps(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw) {
+  const StArg<double, D> S = st_arg<double, D>(A);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
+  const size_t n = (size_t)A->n;
+  const int grid = (M.cols + kThreads - 1) / kThreads;
+  const int group = (int)std::max<size_t>(1, std::min<size_t>((size_t)nvec, kStColsBytes / (16 * n)));
+  const int ng = (nvec + group - 1) / group, G = (nvec + ng - 1) / ng;
+  const int chunk = std::min(steps, 16);  // steps whose sums are added up together
+  const size_t n_part = std::max((size_t)chunk * 3 * G * grid, (size_t)G * kNormBlocks);
+  double *w = (double *)evslcu_malloc(sizeof(double) * (2 * n * G + n_part));
+  if (!w) return EVSLCU_ERR_NOMEM;
+  double *part = w + 2 * n * G;
+  constexpr int J2 = D <= 9 ? 2 : 1;
+  int rc = 0;
+  for (int p0 = 0; p0 < nvec && !rc; p0 += G) {
+    const int nb = std::min(G, nvec - p0);
+    // V[0] starts as the unit probes; w_k+1 takes the place of w_k-1
+    double *V[2] = {w, w + n * nb};
+    const double *x = probes + (size_t)p0 * n;
+    k_st_sumsq<<<dim3(kNormBlocks, nb), kThreads, 0, stream()>>>(A->n, x, part);
+    k_st_unit<<<dim3(std::min(grid_for(A->n), 1024), nb), kThreads, 0, stream()>>>(A->n, x, part, V[0]);
+    count_launch(2);
+    rc = check_launch("k_st_unit");
+    for (int k = 0; k < steps && !rc; ++k) {
+      const double t = (k == 0 ? 1.0 : 2.0) / wid;
+      double *const pk = part + (size_t)(k % chunk) * 3 * nb * grid;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(grid, nb);
+      cfg.blockDim = dim3(kThreads);
+      cfg.stream = stream();
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      // the first step after the scaling, or after sums that still read the
+      // buffer, waits for the whole launch before it
+      attr[0].val.programmaticStreamSerializationAllowed = k % chunk != 0;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      auto fn = M.J == 2 ? (k == 0 ? k_st_kpm<D, J2, true> : k_st_kpm<D, J2, false>)
+                         : (k == 0 ? k_st_kpm<D, 1, true> : k_st_kpm<D, 1, false>);
+      cudaError_t e = cudaLaunchKernelEx(&cfg, fn, S, M, (const double *)V[k % 2], (const double *)V[(k + 1) % 2],
+                                         V[(k + 1) % 2], t, -ctr, pk);
+      rc = e == cudaSuccess ? 0 : fail(EVSLCU_ERR_CUDA, "KPM launch failed: %s", cudaGetErrorString(e));
+      count_launch();
+      if (!rc) rc = check_launch("k_st_kpm");
+      if (!rc && (k % chunk == chunk - 1 || k == steps - 1)) {
+        const int k0 = k - k % chunk, cnt = k % chunk + 1;
+        // (the third sum exists at the first step only; its other places are
+        // not read afterwards)
+        k_st_kpm_sum<<<dim3(nb, 3 * cnt), kThreads, 0, stream()>>>(grid, part, raw + (size_t)k0 * 3 * nvec + p0, nvec);
+        count_launch();
+        rc = check_launch("k_st_kpm_sum");
+      }
+    }
+  }
+  evslcu_free(w);
+  return rc;
+}
+
+template <int D>
+int kpm_d(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw) {
+  if constexpr (D <= kClMaxD) {
+    bool done = false;
+    if (g_cl_force >= 0) {
+      const int rc = kpm_cluster<D>(A, steps, nvec, probes, ctr, wid, raw, &done);
+      if (rc || done) return rc;
+    }
+  }
+  return kpm_steps<D>(A, steps, nvec, probes, ctr, wid, raw);
 }
 
 }  // namespace
@@ -919,8 +1540,8 @@ bool stencil_ok(const evslcu_mat *M) { return M->st_d > 0 && M->use_pat && M->ke
 // variants).
 int stencil_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y,
                  double t, double ncc, double s, double mu0, const evslcu_cheb_epi *epi) {
-  StY Y{first ? 2 : 1, first ? 1 : 0, 0.0, mu0, s};
-  return st_step_any(A, first, vk, vkm1, out, y, t, ncc, Y, epi);
+  StY<double> Y{first ? 2 : 1, first ? 1 : 0, 0.0, mu0, s};
+  return st_step_any(A, first, vk, vkm1, out, y, t, ncc, Y, epi != nullptr, epi);
 }
 
 int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,
@@ -935,7 +1556,7 @@ int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, do
   for (int k = 1; k <= deg; ++k) {
     const double *vk = (k == 1) ? v : W[(k - 2) % 2];
     const double *vkm1 = (k == 1) ? nullptr : ((k == 2) ? v : W[(k - 1) % 2]);
-    StY Y{0, 0, 0.0, 0.0, 0.0};
+    StY<double> Y{0, 0, 0.0, 0.0, 0.0};
     if (k == deg || k - from == 2) {
       Y.terms = k - from + 1;
       Y.init = from == 0;
@@ -944,11 +1565,102 @@ int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, do
       if (Y.terms == 3) Y.c2 = mu[k - 2];
       from = k + 1;
     }
-    const int rc = st_step_any(A, k == 1, vk, vkm1, W[(k - 1) % 2], y, (k == 1) ? t1 : t2, ncc, Y,
+    const int rc = st_step_any(A, k == 1, vk, vkm1, W[(k - 1) % 2], y, (k == 1) ? t1 : t2, ncc, Y, k == deg,
                                k == deg ? epi : nullptr);
     if (rc) return rc;
   }
   return 0;
+}
+
+// Raw sums of the KPM recurrence (sparse.cu, kpm_dots_doubling): raw[(k * 3 +
+// sum) * nvec + probe], on the device.
+int stencil_kpm(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw) {
+  switch (st_width(A->st_d)) {
+    case 5: return kpm_d<5>(A, steps, nvec, probes, ctr, wid, raw);
+    case 7: return kpm_d<7>(A, steps, nvec, probes, ctr, wid, raw);
+    case 9: return kpm_d<9>(A, steps, nvec, probes, ctr, wid, raw);
+    case 16: return kpm_d<16>(A, steps, nvec, probes, ctr, wid, raw);
+    default: return kpm_d<32>(A, steps, nvec, probes, ctr, wid, raw);
+  }
+}
+
+// Whether filter_columns takes these columns: a merged stencil, every degree
+// at least 1.
+bool stencil_columns_ok(const evslcu_mat *A, int ncols, const evslcu_filter_col *cols) {
+  if (!stencil_ok(A)) return false;
+  for (int c = 0; c < ncols; ++c)
+    if (cols[c].deg < 1) return false;
+  return true;
+}
+
+// Device copy of the columns' coefficients, one after another (columns that
+// share an array share its copy); off: each column's first.
+double *stencil_columns_mu(int ncols, const evslcu_filter_col *cols, size_t *off, int *err) {
+  size_t total = 0;
+  for (int c = 0; c < ncols; ++c) {
+    const bool same = c > 0 && cols[c].mu == cols[c - 1].mu && cols[c].deg == cols[c - 1].deg;
+    off[c] = same ? off[c - 1] : total;
+    if (!same) total += (size_t)cols[c].deg + 1;
+  }
+  std::vector<double> h(total);
+  for (int c = 0; c < ncols; ++c) memcpy(h.data() + off[c], cols[c].mu, sizeof(double) * ((size_t)cols[c].deg + 1));
+  double *d = (double *)evslcu_malloc(sizeof(double) * total);
+  *err = d ? evslcu_h2d_async(d, h.data(), sizeof(double) * total)
+           : fail(EVSLCU_ERR_NOMEM, "filter coefficients: out of device memory");
+  if (*err) {
+    evslcu_free(d);
+    return nullptr;
+  }
+  return d;
+}
+
+// The columns' filters; dmu, off from stencil_columns_mu.  work: 4 vectors of
+// n values for min(ncols, 16) columns.
+int stencil_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, const double *dmu,
+                    const size_t *off, void *work) {
+  std::vector<ClMany> many((size_t)ncols);
+  for (int c = 0; c < ncols; ++c)
+    many[c] = ClMany{A, dmu + off[c], cols[c].deg, cols[c].cc, cols[c].dd, cols[c].x, cols[c].y};
+  const size_t vb = fp32 ? sizeof(float) : sizeof(double);
+  if (cl_columns_pay(A, vb, ncols)) return fp32 ? cl_many<float>(ncols, many.data()) : cl_many<double>(ncols, many.data());
+  const size_t per = 4 * vb * (size_t)A->n;
+  const int group = (int)std::max<size_t>(1, std::min<size_t>(kStCols, kStColsBytes / per));
+  // groups of nearly equal size
+  const int ng = (ncols + group - 1) / group;
+  for (int g = 0, c0 = 0; g < ng; ++g) {
+    const int nc = (ncols - c0 + (ng - g) - 1) / (ng - g);
+    const int rc = fp32 ? st_cols_group<float>(A, nc, many.data() + c0, (float *)work)
+                        : st_cols_group<double>(A, nc, many.data() + c0, (double *)work);
+    if (rc) return rc;
+    c0 += nc;
+  }
+  return 0;
+}
+
+// Microseconds of a degree of n columns, from those figures.
+double stencil_step_us(const evslcu_mat *A, int fp32, int n) {
+  double us = 0.0;
+  cl_columns_pay(A, fp32 ? sizeof(float) : sizeof(double), n, &us);
+  return us;
+}
+
+// Takes the columns of an engine's batch that fit a cluster out of it: filters
+// them and marks them in done.
+int stencil_batch(int ncols, const evslcu_batch_col *cols, unsigned char *done) {
+  std::vector<ClMany> many;
+  if (g_cl_force >= 0)
+    for (int c = 0; c < ncols; ++c) {
+      const evslcu_batch_col &b = cols[c];
+      if (!stencil_ok(b.A) || b.deg < 1 || !cl_columns_pay(b.A, sizeof(double), ncols)) continue;
+      many.push_back(ClMany{b.A, b.mu, b.deg, b.cc, b.dd, b.x, b.y});
+      done[c] = 1;
+    }
+  if (many.empty()) return 0;
+  // long filters first: a launch of more clusters than run at once ends sooner
+  std::stable_sort(many.begin(), many.end(),
+                   [](const ClMany &p, const ClMany &q) { return (double)p.deg * p.A->n > (double)q.deg * q.A->n; });
+  std::stable_partition(many.begin(), many.end(), [](const ClMany &p) { return st_mask_bytes(p.A->st_d) == 1; });
+  return cl_many<double>((int)many.size(), many.data());
 }
 
 }  // namespace evslcu

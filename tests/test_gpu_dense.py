@@ -99,3 +99,26 @@ def test_mma_gemm_matches(gpu_lib, m, n, k, pad, beta):
     assert np.max(np.abs(got[:, :m].T - ref)) <= 1e-13 * scale
     assert np.max(np.abs(got - dfma)) <= 1e-13 * scale
     assert np.array_equal(got[:, m:], C0[:, m:])
+
+
+@pytest.mark.parametrize("n, k", [(1, 1), (255, 7), (1025, 130), (40000, 17), (40001, 129), (80001, 33), (160001, 16),
+                                 (3000, 2100)])
+def test_gemv_of_every_column_split(gpu_lib, n, k):
+    """y += A x and y = A^T x (the two products of a Gram-Schmidt pass) at the
+    sizes where the split of the columns changes.  Either order of summation is
+    within (k + 2) eps, or (n + 2) eps, times the sum of absolute products."""
+    rng = np.random.default_rng(n + k)
+    A = rng.standard_normal((k, n))  # column-major n x k
+    x, y, z = rng.standard_normal(k), rng.standard_normal(n), rng.standard_normal(n)
+    lib = gpu_lib.lib
+    dA, dx, dy, dz = (evsl_b200.DeviceBuffer.from_host(lib, v) for v in (A, x, y, z))
+    dh = evsl_b200.DeviceBuffer(lib, 8 * k)
+    ci = lambda v: C.byref(C.c_int(v))  # noqa: E731
+    cd = lambda v: C.byref(C.c_double(v))  # noqa: E731
+    lib.evsl_dgemv_device(b"N", ci(n), ci(k), cd(-1.0), C.c_void_p(dA.ptr), ci(n), C.c_void_p(dx.ptr), ci(1), cd(1.0),
+                          C.c_void_p(dy.ptr), ci(1))
+    lib.evsl_dgemv_device(b"T", ci(n), ci(k), cd(1.0), C.c_void_p(dA.ptr), ci(n), C.c_void_p(dz.ptr), ci(1), cd(0.0),
+                          C.c_void_p(dh.ptr), ci(1))
+    eps = np.finfo(float).eps
+    assert np.all(np.abs(dy.to_host() - (y - x @ A)) <= 2 * (k + 2) * eps * (np.abs(y) + np.abs(x) @ np.abs(A)))
+    assert np.all(np.abs(dh.to_host() - A @ z) <= 2 * (n + 2) * eps * (np.abs(A) @ np.abs(z)))

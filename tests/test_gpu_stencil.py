@@ -117,3 +117,91 @@ def test_dictionaries_that_do_not_merge_keep_the_other_kernels(gpu_lib):
         v = O.seeded_normal(2000, 3)
         pol, mu = polynomial(gpu_lib, 7, 8.0)
         assert np.array_equal(gpu_lib.chebav(pol, v), O.cheb_av(pol.as_dict(), *m, v))
+
+
+MULTI = ["cluster-over", "dropped-7", "eleven", "box-9", "lopsided", "two-rows-5", "two-rows-dropped"]
+
+
+@pytest.mark.parametrize("blocks", [-1, 0])
+@pytest.mark.parametrize("prec", [E.PREC_FP64, E.PREC_MIXED])
+@pytest.mark.parametrize("shape", MULTI)
+def test_stencil_columns_are_bitwise(gpu_lib, shape, prec, blocks):
+    """Several columns with their own polynomials (degrees 1 to 9, so that
+    columns end at different launches; 17 columns: two groups) equal the
+    interleaved SELL-32 kernel's, in both precisions."""
+    n, entries, drop = SHAPES[shape]
+    gpu_lib.set_csr(*stencil_csr(n, entries, drop))
+    bound = max(max(abs(v) for _, v in entries) * len(entries), 1.0)
+    ncols = 17 if n < 20000 else 5
+    X = O.seeded_normal(n * ncols, 4).reshape(ncols, n)
+    made = [polynomial(gpu_lib, 1 + (5 * c) % 9, bound) for c in range(ncols)]
+    pols = [p for p, _ in made]
+    try:
+        gpu_lib.lib.evslcu_set_stencil_cluster(blocks)
+        Y = gpu_lib.chebav_multi(pols, X, prec)
+        gpu_lib.set_filter_variant(0)
+        assert np.array_equal(Y, gpu_lib.chebav_multi(pols, X, prec))
+    finally:
+        gpu_lib.set_filter_variant(-1)
+        gpu_lib.lib.evslcu_set_stencil_cluster(0)
+
+
+def test_engine_batch_of_stencils_of_all_widths(gpu_lib):
+    """Operators with masks of one and of two bytes, with and without a cluster,
+    in one engine: the same eigenvalues as with each matrix's own filter."""
+    box = [(o, -1.0 if o else 8.5) for o, _ in box9(33)]
+    five = [(-40, -1.0), (-1, -1.0), (0, 4.2), (1, -1.0), (40, -1.0)]
+    seven = [(-300, -1.0), (-17, -1.0), (-1, -1.0), (0, 6.4), (1, -1.0), (17, -1.0), (300, -1.0)]
+    wide = [(o, -0.1 if o else 2.0) for o in range(-6, 7)]
+    ops = [(1103, box, 16.5), (2000, five, 8.2), (5001, seven, 12.4), (900, wide, 3.2), (700, five, 8.2), (1500, box, 16.5)]
+    mats = [gpu_lib.matrix(*stencil_csr(n, e)) for n, e, _ in ops]
+    iv = [[0.30 * top, 0.31 * top, 0.0, top] for _, _, top in ops]
+    pols = [gpu_lib.find_pol(i, max_deg=300) for i in iv]
+    out = []
+    for batch in (True, False):
+        eng = gpu_lib.engine(len(ops), precision=E.PREC_FP64)
+        eng.use_batch(batch)
+        for t, (n, _, _) in enumerate(ops):
+            eng.submit_slice(mats[t], iv[t], pols[t], 120, 1e-8, O.seeded_normal(n, t), t)
+        eng.run()
+        got = {}
+        while (r := eng.pop()) is not None:
+            got[r["tag"]] = r["lam"]
+        eng.free()
+        out.append(got)
+    assert len(out[0]) == len(ops)
+    for t in out[0]:
+        assert np.array_equal(out[0][t], out[1][t]), t
+    for m in mats:
+        m.free()
+    for p in pols:
+        gpu_lib.free_pol(p)
+
+
+@pytest.mark.parametrize("blocks", [-1, 0, 1])
+@pytest.mark.parametrize("shape", ["one-row", "tridiagonal", "cluster-over", "cluster-loop", "dropped-7", "eleven",
+                                   "box-9", "two-rows-7"])
+def test_kpm_on_stencils(gpu_lib, shape, blocks):
+    """KPM sums on a merged stencil agree with the CSR kernel's to the rounding
+    of sums of n products of unit vectors (|dots| <= 1: n eps, times 2 for the
+    product identity and 2 for either side), and a probe's do not depend on
+    the probes beside it."""
+    n, entries, drop = SHAPES[shape]
+    m = stencil_csr(n, entries, drop)
+    bound = max(max(abs(v) for _, v in entries) * len(entries), 1.0)
+    iv, M, nvec = [-0.2 * bound, 0.4 * bound, -bound, bound], 21, 7
+    X = O.seeded_normal(n * nvec, 6).reshape(nvec, n)
+    try:
+        gpu_lib.lib.evslcu_set_stencil_cluster(blocks)
+        gpu_lib.set_csr(*m)
+        got = gpu_lib.kpm_dots(M, iv, E.DeviceBuffer.from_host(gpu_lib.lib, X), nvec)
+        parts = [gpu_lib.kpm_dots(M, iv, E.DeviceBuffer.from_host(gpu_lib.lib, np.ascontiguousarray(X[a:b])), b - a)
+                 for a, b in ((0, 1), (1, 6), (6, 7))]
+        assert np.array_equal(got, np.concatenate(parts, axis=1))
+        gpu_lib.set_row_patterns(False)
+        gpu_lib.set_csr(*m)
+        ref = gpu_lib.kpm_dots(M, iv, E.DeviceBuffer.from_host(gpu_lib.lib, X), nvec)
+        assert np.max(np.abs(got - ref)) <= max(4 * n, 1000) * np.finfo(float).eps
+    finally:
+        gpu_lib.set_row_patterns(True)
+        gpu_lib.lib.evslcu_set_stencil_cluster(0)
