@@ -256,7 +256,8 @@ template <int D, int J, bool FIRST>
 __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
     k_st_kpm(const __grid_constant__ StArg<double, D> A, StMarch M, const double *__restrict__ vk, const double *vkm1,
              double *out, double t, double ncc, double *part) {
-  __shared__ double sh[kThreads / 32];
+  constexpr int NS = FIRST ? 3 : 2, NW = kThreads / 32;
+  __shared__ double sh[NS][NW];
   const long long at = (long long)blockIdx.y * A.n;
   double s[3] = {0.0, 0.0, 0.0};
   const StY<double> Y{0, 0, 0.0, 0.0, 0.0};
@@ -266,10 +267,20 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
                                         s[1] += w * x;
                                         if (FIRST) s[2] += x * x;
                                       });
+  // one barrier for all the sums (block_sum's two each kept the warps of a
+  // block waiting a third of the time)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < (FIRST ? 3 : 2); ++q) {
-    const double b = block_sum(s[q], sh);
-    if (threadIdx.x == 0) part[((long long)q * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = b;
+  for (int q = 0; q < NS; ++q) {
+    s[q] = warp_sum(s[q]);
+    if (lane == 0) sh[q][warp] = s[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < NS) {
+    double b = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) b += sh[threadIdx.x][w];
+    part[((long long)threadIdx.x * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = b;
   }
 }
 
@@ -1247,8 +1258,10 @@ int st_cols_launch(const evslcu_mat *A, int na, const StStepCols<VT> &C, int k) 
 }
 
 // Bytes of recurrence vectors that a group of columns may have at once: they
-// stay in L2 from degree to degree.
-constexpr size_t kStColsBytes = (size_t)80 << 20;
+// stay in L2 from degree to degree.  (8 FP64 columns of 343 thousand rows, 100
+// degrees: 2.59 ms in groups of 17 MB, 1.98 of 33, 1.82 of 64, 1.66 in one of 88;
+// KPM of 10^6 rows gains up to 64 MB and loses 3% at 100.)
+constexpr size_t kStColsBytes = (size_t)90 << 20;
 
 // nc (at most kStCols) columns of A, one launch per degree; work: 4 vectors of
 // n VT per column.
