@@ -28,10 +28,13 @@ int evslx_kpm_accumulate(int Mdeg, int damping, int nvec, int n, double *intv, c
   const double beta1 = acos(t);
   t = evsl_min(1.0 - DBL_EPSILON, (bb - ctr) / wid);
   const double beta2 = acos(t);
-  double *jac = (double *)malloc(sizeof(double) * ((size_t)Mdeg + 1));
+  double *jac = (double *)malloc(sizeof(double) * (2 * (size_t)Mdeg + 1));
   if (!jac) return evsl_seterr(EVSLX_ERR_NOMEM, "kpmdos: out of memory");
   dampcf(Mdeg, damping, jac);
   jac[0] = 1.0;
+  /* the sine differences of the count, the same for every probe */
+  double *sdiff = jac + Mdeg + 1;
+  for (int k = 0; k < Mdeg; k++) sdiff[k] = sin((k + 1) * beta2) - sin((k + 1) * beta1);
   memset(mu, 0, sizeof(double) * ((size_t)Mdeg + 1));
   double tcnt = 0.0;
   for (int m = 0; m < nvec; m++) {
@@ -41,7 +44,7 @@ int evslx_kpm_accumulate(int Mdeg, int damping, int nvec, int n, double *intv, c
       const int k1 = k + 1;
       const double tk = 2 * jac[k1] * dots[(size_t)k * nvec + m];
       mu[k1] += tk;
-      tcnt -= tk * (sin(k1 * beta2) - sin(k1 * beta1)) / k1;
+      tcnt -= tk * sdiff[k] / k1;
     }
   }
   t = 1.0 / (((double)nvec) * EVSL_PI);
