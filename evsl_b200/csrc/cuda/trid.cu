@@ -14,6 +14,7 @@
 // q_j = (d_j - x) - e_{j-1}^2 / q_{j-1} with tiny pivots replaced by -pivmin.
 #include <algorithm>
 #include <cfloat>
+#include <cstdint>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -70,6 +71,151 @@ __global__ void __launch_bounds__(kTridThreads)
   }
   if (lane == 0) w[i] = 0.5 * (lo + hi);
 }
+
+// Inverse iteration for eigenvectors j0 .. j0 + m - 1 of T (shift j in
+// shift[j]): one thread per vector, the arithmetic of the host's
+// (invit_range, host/tridiag.c) operation for operation, so the vectors are
+// the same bit for bit.  A vector is a chain of a few thousand dependent
+// divisions and updates that costs the host 60 us at 850 rows; here all of them
+// run side by side, and what bounds it is one chain.  Arrays are [row][vector],
+// so that a warp's accesses are contiguous; rows are taken eight at a time
+// with their loads issued before the chain needs them.
+constexpr int kInvitIters = 3;
+
+struct InvitWork {
+  double *u0, *u1, *u2, *ml, *x;
+  unsigned char *swp;
+};
+
+__device__ __forceinline__ double invit_start(uint64_t j, uint64_t i) {
+  uint64_t z = (j << 32) + i;
+  z += 0x9E3779B97F4A7C15ULL;
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+  z ^= z >> 31;
+  return __dadd_rn(__dmul_rn((double)(z >> 11), 1.0 / 9007199254740992.0), -0.5);
+}
+
+__global__ void __launch_bounds__(32)
+    k_trid_invit(int n, int m, int j0, const double *__restrict__ d, const double *__restrict__ e,
+                 const double *__restrict__ shift, double tiny, InvitWork W, double *__restrict__ Z, long long ldz) {
+  constexpr int U = 8;
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  if (c >= m) return;
+  const size_t M = (size_t)m;
+  const double lam = shift[j0 + c];
+  double *const u0 = W.u0 + c, *const u1 = W.u1 + c, *const u2 = W.u2 + c, *const ml = W.ml + c, *const x = W.x + c;
+  unsigned char *const swp = W.swp + c;
+  auto floor_tiny = [&](double v) { return fabs(v) < tiny ? (v < 0.0 ? -tiny : tiny) : v; };
+  // LU with partial pivoting of T - lam I: dg, du are rows i's entries so far
+  {
+    double dg = __dadd_rn(__ldg(d), -lam), du = n > 1 ? __ldg(e) : 0.0;
+    for (int i = 0; i < n - 1; ++i) {
+      const double sub = __ldg(e + i), dn = __dadd_rn(__ldg(d + i + 1), -lam), un = (i < n - 2) ? __ldg(e + i + 1) : 0.0;
+      const size_t at = (size_t)i * M;
+      if (fabs(dg) >= fabs(sub)) {
+        const double l = (dg != 0.0) ? __ddiv_rn(sub, dg) : 0.0;
+        u0[at] = floor_tiny(dg);
+        u1[at] = du;
+        u2[at] = 0.0;
+        ml[at] = l;
+        swp[at] = 0;
+        dg = __dadd_rn(dn, -__dmul_rn(l, du));
+        du = un;
+      } else {
+        const double l = __ddiv_rn(dg, sub);
+        u0[at] = floor_tiny(sub);
+        u1[at] = dn;
+        u2[at] = un;
+        ml[at] = l;
+        swp[at] = 1;
+        dg = __dadd_rn(du, -__dmul_rn(l, dn));
+        du = (i < n - 2) ? __dmul_rn(-l, un) : un;
+      }
+    }
+    u0[(size_t)(n - 1) * M] = floor_tiny(dg);
+  }
+  for (int i = 0; i < n; ++i) x[(size_t)i * M] = invit_start((uint64_t)(j0 + c), (uint64_t)i);
+  for (int it = 0; it < kInvitIters; ++it) {
+    // forward: P L (xi: row i's value so far)
+    double xi = x[0];
+    for (int b = 0; b < n - 1; b += U) {
+      double l[U], xn[U];
+      unsigned char sw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t at = (size_t)min(b + u, n - 2) * M;
+        l[u] = ml[at];
+        sw[u] = swp[at];
+        xn[u] = x[at + M];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b + u < n - 1) {
+          const double lo = sw[u] ? xn[u] : xi, hi = sw[u] ? xi : xn[u];
+          x[(size_t)(b + u) * M] = lo;
+          xi = __dadd_rn(hi, -__dmul_rn(l[u], lo));
+        }
+    }
+    // back: U
+    double amax = 0.0, x1 = __ddiv_rn(xi, u0[(size_t)(n - 1) * M]), x2 = 0.0;  // x1, x2: rows i + 1, i + 2
+    x[(size_t)(n - 1) * M] = x1;
+    for (int b = n - 2; b >= 0; b -= U) {
+      double p0[U], p1[U], p2[U], xr[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t at = (size_t)max(b - u, 0) * M;
+        p0[u] = u0[at];
+        p1[u] = u1[at];
+        p2[u] = u2[at];
+        xr[u] = x[at];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b - u >= 0) {
+          double t = __dadd_rn(xr[u], -__dmul_rn(p1[u], x1));
+          if (b - u < n - 2) t = __dadd_rn(t, -__dmul_rn(p2[u], x2));
+          t = __ddiv_rn(t, p0[u]);
+          x[(size_t)(b - u) * M] = t;
+          x2 = x1;
+          x1 = t;
+        }
+    }
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) {
+      const double v = fabs(x[(size_t)i * M]);
+      amax = amax > v ? amax : v;
+    }
+    if (amax == 0.0) {
+      x[(size_t)((j0 + c) % n) * M] = 1.0;
+      amax = 1.0;
+    }
+    double nrm = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) {
+      const double v = __ddiv_rn(x[(size_t)i * M], amax);
+      x[(size_t)i * M] = v;
+      nrm = __dadd_rn(nrm, __dmul_rn(v, v));
+    }
+    nrm = __dsqrt_rn(nrm);
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) x[(size_t)i * M] = __ddiv_rn(x[(size_t)i * M], nrm);
+  }
+  // sign convention: largest component (the first of equals) positive
+  double big = x[0];
+#pragma unroll 8
+  for (int i = 1; i < n; ++i) {
+    const double v = x[(size_t)i * M];
+    if (fabs(v) > fabs(big)) big = v;
+  }
+  const double sgn = big < 0.0 ? -1.0 : 1.0;
+  double *z = Z + (long long)(j0 + c) * ldz;
+#pragma unroll 8
+  for (int i = 0; i < n; ++i) z[i] = __dmul_rn(sgn, x[(size_t)i * M]);
+}
+
+// Scratch of a launch at most; more vectors go in several.
+constexpr size_t kInvitBytes = (size_t)512 << 20;
 
 double *g_trid_buf = nullptr;
 int g_trid_cap = 0;
@@ -253,6 +399,31 @@ int evslcu_trid_eigvals_async_wait(double *w) {
   for (int i = 0; i < i0; ++i) w[i] = g_async.glo;
   std::sort(w, w + k);
   return 0;
+}
+
+int evslcu_trid_invit(int n, const double *d, const double *e, int m, const double *shift, double tiny, double *Z,
+                      long long ldz) {
+  if (n < 2 || m < 1 || !d || !e || !shift || !Z) return fail(EVSLCU_ERR_ARG, "trid_invit: bad arguments");
+  const size_t row = 5 * sizeof(double) + 1;
+  const int chunk = (int)std::max<size_t>(32, std::min<size_t>((size_t)m, kInvitBytes / (row * (size_t)n)));
+  const int mc = std::min(m, chunk);
+  const size_t in = (size_t)2 * n + m;
+  double *buf = (double *)evslcu_malloc(sizeof(double) * in + row * (size_t)n * mc);
+  if (!buf) return EVSLCU_ERR_NOMEM;
+  double *dd = buf, *de = buf + n, *ds = buf + 2 * (size_t)n, *w = buf + in;
+  int rc = evslcu_h2d_async(dd, d, sizeof(double) * (size_t)n);
+  if (!rc) rc = evslcu_h2d_async(de, e, sizeof(double) * (size_t)(n - 1));
+  if (!rc) rc = evslcu_h2d_async(ds, shift, sizeof(double) * (size_t)m);
+  const size_t blk = (size_t)n * mc;
+  const InvitWork W{w, w + blk, w + 2 * blk, w + 3 * blk, w + 4 * blk, (unsigned char *)(w + 5 * blk)};
+  for (int j0 = 0; j0 < m && !rc; j0 += mc) {
+    const int c = std::min(mc, m - j0);
+    k_trid_invit<<<(c + 31) / 32, 32, 0, stream()>>>(n, c, j0, dd, de, ds, tiny, W, Z, ldz);
+    count_launch();
+    rc = check_launch("k_trid_invit");
+  }
+  evslcu_free(buf);
+  return rc;
 }
 
 int evslcu_trid_eigvals(int k, const double *d, const double *e, double *w) {

@@ -387,6 +387,12 @@ int evslcu_trid_eigvals_above(int k, const double *d, const double *e, double xm
 int evslcu_trid_eigvals_async(int k, const double *d, const double *e, double xmin);
 int evslcu_trid_eigvals_async_ready(void);
 int evslcu_trid_eigvals_async_wait(double *w);
+/* Eigenvectors by inverse iteration at the m shifts (ascending, on the host, as
+ * d and e) of the symmetric tridiagonal matrix, into the columns of Z (device,
+ * leading dimension ldz): the host's arithmetic, one thread per vector, no
+ * orthogonalisation among them. */
+int evslcu_trid_invit(int n, const double *d, const double *e, int m, const double *shift, double tiny, double *Z,
+                      long long ldz);
 /* Pattern tables read from the constant-memory pool when they fit there (1,
  * default) or always from global memory (0).  Same arithmetic either way. */
 int evslcu_set_pattern_const(int on);

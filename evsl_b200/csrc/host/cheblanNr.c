@@ -87,7 +87,7 @@ int ChebLanNr(double *intv, int maxit, double tol, double *vinit, polparams *pol
   double *dT = (double *)malloc(sizeof(double) * (size_t)maxit);
   double *eT = (double *)malloc(sizeof(double) * (size_t)maxit);
   double *EvalT = (double *)malloc(sizeof(double) * (size_t)maxit);
-  double *Lam = NULL, *res = NULL, *Rvec = NULL, *W = NULL, *EvecT = NULL, *EvecT_dev = NULL;
+  double *Lam = NULL, *res = NULL, *Rvec = NULL, *W = NULL, *EvecT_dev = NULL;
   double *rnorm = NULL, *rlam = NULL, *rres = NULL;
   int *sel = NULL;
   int kdim = 0, count = 0, nev = 0;
@@ -217,13 +217,13 @@ int ChebLanNr(double *intv, int maxit, double tol, double *vinit, polparams *pol
     evslh.last_candidates = msel;
     double *wsel = (double *)malloc(sizeof(double) * (size_t)(msel > 0 ? msel : 1));
     for (int j = 0; j < msel; j++) wsel[j] = EvalT[sel[j]];
-    EvecT = (double *)malloc(sizeof(double) * (size_t)kdim * (size_t)(msel > 0 ? msel : 1));
-    if (!EvecT) {
+    if (msel > 0) EvecT_dev = (double *)evslcu_malloc(sizeof(double) * (size_t)kdim * msel);
+    if (msel > 0 && !EvecT_dev) {
       free(wsel);
       rc = evsl_seterr(EVSLX_ERR_NOMEM, "ChebLanNr: out of memory (Ritz)");
       goto done;
     }
-    rc = evsl_trid_eigvecs(kdim, dT, eT, msel, wsel, EvecT, kdim);
+    rc = evsl_trid_eigvecs_device(kdim, dT, eT, msel, wsel, EvecT_dev);
     free(wsel);
     if (rc) goto done;
     evslstat.t_eig += evsl_timer() - te;
@@ -231,17 +231,15 @@ int ChebLanNr(double *intv, int maxit, double tol, double *vinit, polparams *pol
     Lam = (double *)malloc(sizeof(double) * (size_t)(msel > 0 ? msel : 1));
     res = (double *)malloc(sizeof(double) * (size_t)(msel > 0 ? msel : 1));
     if (msel > 0) {
-      EvecT_dev = (double *)evslcu_malloc(sizeof(double) * (size_t)kdim * msel);
       Rvec = (double *)evslcu_malloc(sizeof(double) * n_l * msel);
       W = (double *)evslcu_malloc(sizeof(double) * n_l * msel);
       rnorm = (double *)malloc(sizeof(double) * 3 * (size_t)msel);
-      if (!EvecT_dev || !Rvec || !W || !rnorm || !Lam || !res) {
+      if (!Rvec || !W || !rnorm || !Lam || !res) {
         rc = evsl_seterr(EVSLX_ERR_NOMEM, "ChebLanNr: out of memory for %d Ritz vectors", msel);
         goto done;
       }
       rlam = rnorm + msel;
       rres = rlam + msel;
-      if ((rc = evslcu_h2d(EvecT_dev, EvecT, sizeof(double) * (size_t)kdim * msel))) goto cuda_fail;
       /* Rvec = V(:, 1:kdim) * EvecT(:, sel) */
       if ((rc = evslcu_dgemm('N', 'N', n, msel, kdim, 1.0, V, n, EvecT_dev, kdim, 0.0, Rvec, n))) goto cuda_fail;
       if ((rc = evslcu_ritz_eval(op, n, msel, Rvec, W, rnorm, rlam, rres))) goto cuda_fail;
@@ -296,7 +294,6 @@ done:
   free(dT);
   free(eT);
   free(EvalT);
-  free(EvecT);
   free(Lam);
   free(res);
   free(rnorm);

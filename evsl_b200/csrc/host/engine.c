@@ -734,7 +734,7 @@ static int finalize(evslx_engine *E, slot_t *s, int kdim, evslx_result *out) {
   int rc = 0, msel = 0, nev = 0;
   int *sel = (int *)malloc(sizeof(int) * (size_t)(kdim > 0 ? kdim : 1));
   double *wsel = (double *)malloc(sizeof(double) * (size_t)(kdim > 0 ? kdim : 1));
-  double *EvecT = NULL, *EvecT_dev = NULL, *Rvec = NULL, *W = NULL, *rnorm = NULL;
+  double *EvecT_dev = NULL, *Rvec = NULL, *W = NULL, *rnorm = NULL;
   int *keep = NULL;
   if (!sel || !wsel) {
     rc = evsl_seterr(EVSLX_ERR_NOMEM, "engine: out of memory");
@@ -767,7 +767,6 @@ static int finalize(evslx_engine *E, slot_t *s, int kdim, evslx_result *out) {
     }
     msel += g;
   }
-  EvecT = (double *)malloc(sizeof(double) * (size_t)kdim * msel);
   EvecT_dev = (double *)evslcu_malloc(sizeof(double) * (size_t)kdim * msel);
   Rvec = (double *)evslcu_malloc(sizeof(double) * n_l * msel);
   W = (double *)evslcu_malloc(sizeof(double) * n_l * msel);
@@ -775,14 +774,13 @@ static int finalize(evslx_engine *E, slot_t *s, int kdim, evslx_result *out) {
   keep = (int *)malloc(sizeof(int) * (size_t)msel);
   out->lam = (double *)malloc(sizeof(double) * (size_t)msel);
   out->res = (double *)malloc(sizeof(double) * (size_t)msel);
-  if (!EvecT || !EvecT_dev || !Rvec || !W || !rnorm || !keep || !out->lam || !out->res) {
+  if (!EvecT_dev || !Rvec || !W || !rnorm || !keep || !out->lam || !out->res) {
     rc = evsl_seterr(EVSLX_ERR_NOMEM, "engine: out of memory for %d Ritz vectors", msel);
     goto done;
   }
   double *rlam = rnorm + msel, *rres = rlam + msel;
-  if ((rc = evsl_trid_eigvecs(kdim, s->dT, s->eT, msel, wsel, EvecT, kdim))) goto done;
-  if ((rc = evslcu_h2d(EvecT_dev, EvecT, sizeof(double) * (size_t)kdim * msel)) ||
-      (rc = evslcu_dgemm('N', 'N', n, msel, kdim, 1.0, s->V, n, EvecT_dev, kdim, 0.0, Rvec, n)) ||
+  if ((rc = evsl_trid_eigvecs_device(kdim, s->dT, s->eT, msel, wsel, EvecT_dev))) goto done;
+  if ((rc = evslcu_dgemm('N', 'N', n, msel, kdim, 1.0, s->V, n, EvecT_dev, kdim, 0.0, Rvec, n)) ||
       (rc = evslcu_ritz_eval(&r->M->op, n, msel, Rvec, W, rnorm, rlam, rres))) {
     rc = evsl_seterr(rc, "%s", evslcu_errstr());
     goto done;
@@ -818,7 +816,6 @@ done:
   out->nev = nev;
   free(sel);
   free(wsel);
-  free(EvecT);
   free(rnorm);
   free(keep);
   evslcu_free(EvecT_dev);

@@ -58,6 +58,7 @@ int evsl_trid_eigvals_test(int n, const double *d, const double *e, double xmin,
 int evsl_trid_test_start(int n, const double *d, const double *e, double xmin);
 int evsl_trid_test_ready(void);
 int evsl_trid_test_wait(double *w);
+int evsl_trid_eigvecs_device(int n, const double *d, const double *e, int m, const double *w, double *Z);
 int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const double *w, double *Z, int ldz);
 int evsl_sym_eig(int n, const double *A, int lda, double *Q, int ldq, double *w);
 int evsl_tr_eig(int k, int m, const double *T, int ldt, double thresh, double *w, double *Z, int ldz);

@@ -15,7 +15,9 @@
  *                      iteration with a pivoted tridiagonal LU and
  *                      re-orthogonalisation inside clusters of close
  *                      eigenvalues (Peters & Wilkinson 1971; the approach
- *                      of LAPACK's dstein), O(n) per vector and iteration.
+ *                      of LAPACK's dstein), O(n) per vector and iteration;
+ *                      evsl_trid_eigvecs_device does it on the GPU, a thread
+ *                      per vector, with the same bits.
  *   evsl_tr_eig        the thick-restart matrix (diagonal block + spike row
  *                      + tridiagonal tail): the leading block is reduced to
  *                      tridiagonal form by a Lanczos run on the diagonal
@@ -207,6 +209,7 @@ typedef struct {
   const double *d, *e, *shift;
   const int *cst;
   double *Z, tiny;
+  int zfirst; /* the vector in Z's first column */
 } invit_job;
 
 static int invit_range(invit_job *jb) {
@@ -276,7 +279,7 @@ static int invit_range(invit_job *jb) {
       /* orthogonalise against the earlier vectors of the cluster (twice) */
       for (int pass = 0; pass < 2 && cstart < j; pass++) {
         for (int q = cstart; q < j; q++) {
-          const double *zq = Z + (size_t)q * ldz;
+          const double *zq = Z + (size_t)(q - jb->zfirst) * ldz;
           double dot = 0.0;
           for (int i = 0; i < n; i++) dot += zq[i] * x[i];
           for (int i = 0; i < n; i++) x[i] -= dot * zq[i];
@@ -300,7 +303,7 @@ static int invit_range(invit_job *jb) {
     for (int i = 1; i < n; i++)
       if (fabs(x[i]) > fabs(x[imax])) imax = i;
     const double sgn = (x[imax] < 0.0) ? -1.0 : 1.0;
-    double *zj = Z + (size_t)j * ldz;
+    double *zj = Z + (size_t)(j - jb->zfirst) * ldz;
     for (int i = 0; i < n; i++) zj[i] = sgn * x[i];
   }
   free(buf);
@@ -317,12 +320,9 @@ static void *invit_thread(void *arg) {
 #define INVIT_MAX_THREADS 16
 #define INVIT_MIN_WORK (1L << 21) /* vectors x rows per thread */
 
-int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const double *w, double *Z, int ldz) {
-  if (m <= 0 || n <= 0) return 0;
-  if (n == 1) {
-    for (int j = 0; j < m; j++) Z[(size_t)j * ldz] = 1.0;
-    return 0;
-  }
+/* Shifts (the eigenvalues, separated by at least pert) and cluster starts of m
+ * ascending eigenvalues; returns the norm of T (1 for T = 0). */
+static double invit_shifts(int n, const double *d, const double *e, int m, const double *w, double *shift, int *cst) {
   double tnorm = 0.0;
   for (int i = 0; i < n; i++) {
     double r = fabs(d[i]);
@@ -333,14 +333,6 @@ int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const doub
   if (tnorm == 0.0) tnorm = 1.0;
   const double pert = 10.0 * DBL_EPSILON * tnorm;
   const double clus = CLUSTER_TOL * tnorm;
-  /* shifts (separated by at least pert) and cluster starts, in order */
-  double *shift = (double *)malloc(sizeof(double) * (size_t)m);
-  int *cst = (int *)malloc(sizeof(int) * (size_t)m);
-  if (!shift || !cst) {
-    free(shift);
-    free(cst);
-    return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-  }
   int cstart = 0;
   double lam_prev = 0.0;
   for (int j = 0; j < m; j++) {
@@ -353,6 +345,71 @@ int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const doub
     shift[j] = lam;
     cst[j] = cstart;
   }
+  return tnorm;
+}
+
+/* evsl_trid_eigvecs with the vectors on the device (Z: n x m, ld n): on the GPU,
+ * bit for bit the host's, except clusters of close eigenvalues, whose vectors
+ * are orthogonalised one after another -- those on the host, then copied. */
+int evsl_trid_eigvecs_device(int n, const double *d, const double *e, int m, const double *w, double *Z) {
+  if (m <= 0 || n <= 0) return 0;
+  if (n < 2) {
+    double *one = (double *)malloc(sizeof(double) * (size_t)m);
+    if (!one) return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+    for (int j = 0; j < m; j++) one[j] = 1.0;
+    const int rc1 = evslcu_h2d(Z, one, sizeof(double) * (size_t)m);
+    free(one);
+    return rc1 ? evsl_seterr(rc1, "%s", evslcu_errstr()) : 0;
+  }
+  double *shift = (double *)malloc(sizeof(double) * (size_t)m);
+  int *cst = (int *)malloc(sizeof(int) * (size_t)m);
+  if (!shift || !cst) {
+    free(shift);
+    free(cst);
+    return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+  }
+  const double tnorm = invit_shifts(n, d, e, m, w, shift, cst);
+  int rc = evslcu_trid_invit(n, d, e, m, shift, DBL_EPSILON * tnorm, Z, n);
+  if (rc) rc = evsl_seterr(rc, "%s", evslcu_errstr());
+  for (int j0 = 0; j0 < m && !rc;) {
+    int j1 = j0 + 1;
+    while (j1 < m && cst[j1] == j0) j1++;
+    if (j1 - j0 > 1) {
+      /* Zc: the cluster's columns, addressed by their numbers in all m */
+      const size_t cnt = (size_t)(j1 - j0) * n;
+      double *Zc = (double *)malloc(sizeof(double) * cnt);
+      if (!Zc) {
+        rc = evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+      } else {
+        invit_job jb = {n, n, j0, j1, 0, d, e, shift, cst, Zc, DBL_EPSILON * tnorm, j0};
+        if (invit_range(&jb))
+          rc = evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+        else if ((rc = evslcu_h2d(Z + (size_t)j0 * n, Zc, sizeof(double) * cnt)))
+          rc = evsl_seterr(rc, "%s", evslcu_errstr());
+        free(Zc);
+      }
+    }
+    j0 = j1;
+  }
+  free(shift);
+  free(cst);
+  return rc;
+}
+
+int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const double *w, double *Z, int ldz) {
+  if (m <= 0 || n <= 0) return 0;
+  if (n == 1) {
+    for (int j = 0; j < m; j++) Z[(size_t)j * ldz] = 1.0;
+    return 0;
+  }
+  double *shift = (double *)malloc(sizeof(double) * (size_t)m);
+  int *cst = (int *)malloc(sizeof(int) * (size_t)m);
+  if (!shift || !cst) {
+    free(shift);
+    free(cst);
+    return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+  }
+  const double tnorm = invit_shifts(n, d, e, m, w, shift, cst);
   /* ranges split at cluster starts over host threads; every vector is
    * computed the same way whatever the split */
   long nth = sysconf(_SC_NPROCESSORS_ONLN);
@@ -364,7 +421,7 @@ int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const doub
     int j1 = (t == nth - 1 || nth <= 1) ? m : (int)(((long)m * (t + 1)) / nth);
     if (j1 < j0 + 1) j1 = j0 + 1;
     while (j1 < m && cst[j1] != j1) j1++;
-    jobs[nj] = (invit_job){n, ldz, j0, j1, 0, d, e, shift, cst, Z, DBL_EPSILON * tnorm};
+    jobs[nj] = (invit_job){n, ldz, j0, j1, 0, d, e, shift, cst, Z, DBL_EPSILON * tnorm, 0};
     nj++;
     j0 = j1;
   }

@@ -122,3 +122,34 @@ def test_gemv_of_every_column_split(gpu_lib, n, k):
     eps = np.finfo(float).eps
     assert np.all(np.abs(dy.to_host() - (y - x @ A)) <= 2 * (k + 2) * eps * (np.abs(y) + np.abs(x) @ np.abs(A)))
     assert np.all(np.abs(dh.to_host() - A @ z) <= 2 * (n + 2) * eps * (np.abs(A) @ np.abs(z)))
+
+
+@pytest.mark.parametrize("n, m, kind", [(1, 1, "random"), (2, 2, "random"), (9, 9, "random"), (70, 33, "random"),
+                                        (515, 257, "random"), (1601, 40, "random"), (64, 64, "split"),
+                                        (400, 90, "clusters")])
+def test_tridiagonal_eigenvectors_on_gpu_are_the_hosts(gpu_lib, n, m, kind):
+    """Inverse iteration with one thread per vector gives the host's vectors bit
+    for bit, those of clusters (done on the host in both) included."""
+    lib = gpu_lib.lib
+    vp = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    for f in (lib.evsl_trid_eigvecs, lib.evsl_trid_eigvecs_device, lib.evsl_trid_eigvals):
+        f.restype = C.c_int
+    lib.evsl_trid_eigvals.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.evsl_trid_eigvecs.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int]
+    lib.evsl_trid_eigvecs_device.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+    rng = np.random.default_rng(n + m)
+    if kind == "clusters":  # four identical blocks: every eigenvalue four times
+        b = n // 4
+        d, e = np.tile(rng.uniform(-0.1, 1.0, b), 4), np.tile(np.r_[rng.uniform(0.01, 0.3, b - 1), 0.0], 4)
+    else:
+        d, e = rng.uniform(-0.1, 1.0, n), rng.uniform(0.01, 0.3, n)
+        if kind == "split":
+            e[n // 2] = 0.0
+    w = np.zeros(n)
+    assert lib.evsl_trid_eigvals(n, vp(d), vp(e), vp(w)) == 0
+    sel = np.ascontiguousarray(w[n - m:])
+    Z = np.zeros((m, n))
+    dZ = evsl_b200.DeviceBuffer(lib, Z.nbytes)
+    assert lib.evsl_trid_eigvecs(n, vp(d), vp(e), m, vp(sel), vp(Z), n) == 0
+    assert lib.evsl_trid_eigvecs_device(n, vp(d), vp(e), m, vp(sel), C.c_void_p(dZ.ptr)) == 0
+    assert np.array_equal(dZ.to_host(shape=Z.shape), Z)
