@@ -752,7 +752,12 @@ __global__ void __launch_bounds__(cl_threads(-1, ONE), 1)
     k_st_clusters(const __grid_constant__ StTab tab, int polls, int *err) {
   const StCol &I = tab.c[blockIdx.x / cluster_size()];
   const double *mup = I.mu;
-  st_cluster_body<VT, D, ONE, true>(I, [&](int k) { return __ldg(mup + k); }, polls, err);
+  auto mu = [&](int k) { return __ldg(mup + k); };
+  // 5- and 7-point operators may be in one launch, each with its own row product
+  if (D == 7 && I.d <= 5)
+    st_cluster_body<VT, 5, ONE, true>(I, mu, polls, err);
+  else
+    st_cluster_body<VT, D, ONE, true>(I, mu, polls, err);
 }
 
 // The whole KPM recurrence of a probe (k_st_kpm's steps, the probe made a unit
@@ -928,7 +933,7 @@ struct ClPlan {
   int cl = 0, R = 0, T = 0, halo = 0, y_smem = 0;
   size_t smem = 0;
 };
-constexpr size_t kClSmemMax = 225 * 1024;
+constexpr size_t kClSmemMax = 224 * 1024;  // of 227 KB, less the static and the reserved part
 
 ClPlan cl_plan(int n, int reach, int d, size_t vb, int cl, int cap) {
   ClPlan P;
@@ -1061,6 +1066,8 @@ template <class VT, int D>
 int cl_launch_many(int ncols, const StTab &tab, int cl, int T, size_t smem, bool one) {
   int *err = cl_err();
   if (!err) return fail(EVSLCU_ERR_NOMEM, "cluster filter: out of pinned host memory");
+  if ((one ? cl_max1<VT, D, -1, true>() : cl_max1<VT, D, -1, false>()) < cl)
+    return fail(EVSLCU_ERR_CUDA, "clusters of %d blocks are not available", cl);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl * ncols);
   cfg.blockDim = dim3(T);
@@ -1094,7 +1101,6 @@ void cl_column(StCol &C, const evslcu_mat *A, int deg, double cc, double dd, con
   C.R = P.R;
   C.halo = P.halo;
   C.y_smem = P.y_smem;
-  // D: the compiled width (of the launch's widest stencil)
   C.full = A->st_d == D ? (1u << D) - 1u : 0xffffffffu;
   C.center = A->st_d == D && A->st_off[D / 2] == 0;
   for (int e = 0; e < A->st_d; ++e) {
@@ -1161,10 +1167,10 @@ struct ClMany {
   double *y;
 };
 
-// Most blocks per cluster of those launches.
+// Most blocks per cluster of those launches (each kernel's own limit is set
+// when it is first launched).
 int cl_many_most(size_t vb) {
-  if (vb == sizeof(float)) return std::min(cl_most<float, -1>(5), std::min(cl_most<float, -1>(7), cl_most<float, -1>(9)));
-  return std::min(cl_most<double, -1>(5), std::min(cl_most<double, -1>(7), cl_most<double, -1>(9)));
+  return vb == sizeof(float) ? cl_max1<float, 7, -1, false>() : cl_max1<double, 7, -1, false>();
 }
 
 // Plan of one column in a launch of cl blocks per column and precision vb.
@@ -1173,9 +1179,43 @@ ClPlan cl_plan_many(const evslcu_mat *A, size_t vb, int cl) {
   return cl_plan(A->n, A->st_reach, A->st_d, vb, cl, -1);
 }
 
+// Microseconds of a degree of one column with that plan (as measured: up to
+// 512 rows a block has one row per thread).
+double cl_degree_us(const evslcu_mat *A, const ClPlan &P) {
+  if (P.R <= 512) return A->st_d <= 5 ? 0.53 : 0.62;
+  return 0.45 + (A->st_d <= 5 ? 0.7e-3 : 1.15e-3) * P.R;
+}
+
+// Clusters of cl blocks that run at once (a block has an SM to itself).
+int cl_slots(int cl) {
+  static int slots[17] = {};
+  if (slots[cl]) return slots[cl];
+  cl_many_most(sizeof(double));  // sets the kernel's limits
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl * sm_count());
+  cfg.blockDim = dim3(cl_threads(-1, false));
+  cfg.dynamicSmemBytes = kClSmemMax;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int got = 0;
+  if (cudaOccupancyMaxActiveClusters(&got, (const void *)k_st_clusters<double, 7, false>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    got = 0;
+  }
+  return slots[cl] = got > 0 ? got : std::max(1, sm_count() / cl / 2);
+}
+
 // Filters n columns (each of which has a plan) in launches of up to kClCols
-// clusters; a launch's operators have masks of one type.  It takes the largest
-// cluster that still lets its columns run at once.
+// clusters; a launch's operators have masks of one type.  Larger clusters make
+// a column faster and let fewer run at once: of the sizes every column fits,
+// the launch takes the one whose columns, each starting where a cluster is
+// free first, are done soonest.  (Sixteen operators of 1,000 to 17,000 rows,
+// degrees 11 to 338: with 8 blocks all run at once and the longest takes 620
+// us; with 16 it takes 400 and the others fit beside it.)
 template <class VT>
 int cl_many(int n, const ClMany *cols) {
   const int most = cl_many_most(sizeof(VT));
@@ -1183,12 +1223,24 @@ int cl_many(int n, const ClMany *cols) {
     nc = 1;
     const int mb = st_mask_bytes(cols[c0].A->st_d);
     while (nc < kClCols && c0 + nc < n && st_mask_bytes(cols[c0 + nc].A->st_d) == mb) ++nc;
-    // the smallest cluster every column fits, then larger while they all run at once
     int cl = 0;
+    double best = 0.0;
     for (int t = 1; t <= most; t *= 2) {
+      std::vector<double> busy((size_t)std::min(nc, cl_slots(t)), 0.0);
+      double end = 0.0;
       bool fits = true;
-      for (int i = 0; i < nc && fits; ++i) fits = cl_plan_many(cols[c0 + i].A, sizeof(VT), t).cl > 0;
-      if (fits && (!cl || t * nc <= sm_count())) cl = t;
+      for (int i = 0; i < nc && fits; ++i) {
+        const ClMany &c = cols[c0 + i];
+        const ClPlan P = cl_plan_many(c.A, sizeof(VT), t);
+        fits = P.cl > 0;
+        auto slot = std::min_element(busy.begin(), busy.end());
+        *slot += c.deg * cl_degree_us(c.A, P);
+        end = std::max(end, *slot);
+      }
+      if (fits && (!cl || end < best)) {
+        cl = t;
+        best = end;
+      }
     }
     if (!cl) return fail(EVSLCU_ERR_ARG, "cluster filter: a column does not fit");
     StTab tab;
@@ -1199,7 +1251,7 @@ int cl_many(int n, const ClMany *cols) {
     for (int i = 0; i < nc; ++i) {
       const ClMany &c = cols[c0 + i];
       const ClPlan P = cl_plan_many(c.A, sizeof(VT), cl);
-      cl_column(tab.c[i], c.A, c.deg, c.cc, c.dd, c.x, c.y, P, D);
+      cl_column(tab.c[i], c.A, c.deg, c.cc, c.dd, c.x, c.y, P, st_width(c.A->st_d));
       tab.c[i].mu = c.mu;
       T = std::max(T, P.T);
       // (a plan of one row per thread has no room for the masks)
@@ -1214,25 +1266,24 @@ int cl_many(int n, const ClMany *cols) {
   return 0;
 }
 
-// Whether n columns of A go to clusters rather than to one launch per degree:
-// most blocks a column may have, and the time of a degree of all columns on
-// either, as measured: on a cluster 0.45 us plus 0.7 (5-point) or 1.15 us per
-// thousand rows of a block above one row per thread; k_st_cols 2.2 us a launch
-// plus 6.3 (FP32: 3.6) us per million rows.
+// Whether n columns of A go to clusters rather than to one launch per degree,
+// by the time of a degree of all of them: cl_degree_us, or for k_st_cols 2.2 us
+// a launch plus 6.3 (FP32: 3.6) us per million rows, as measured.
 bool cl_columns_pay(const evslcu_mat *A, size_t vb, int n, double *us = nullptr) {
   const double step = 2.2 + (vb == 8 ? 6.3e-6 : 3.6e-6) * (double)A->n * n;
   if (us) *us = step;
   if (A->st_d > kClMaxD || g_cl_force < 0) return false;
   const int most = cl_many_most(vb);
-  int cl = 0;
-  for (int t = 1; t <= most; t *= 2)
-    if (cl_plan_many(A, vb, t).cl && (!cl || t * std::min(n, kClCols) <= sm_count())) cl = t;
-  if (!cl) return false;
-  const ClPlan P = cl_plan_many(A, vb, cl);
-  const double deg1 = 0.45 + (P.R > 512 ? (A->st_d <= 5 ? 0.7e-3 : 1.15e-3) * P.R : 0.0);
-  const double waves = std::max(1.0, std::ceil((double)n * cl / sm_count()));
-  if (us) *us = std::min(step, waves * deg1);
-  return g_cl_force > 0 || waves * deg1 < step;
+  double cluster = 0.0;
+  for (int t = 1; t <= most; t *= 2) {
+    const ClPlan P = cl_plan_many(A, vb, t);
+    if (!P.cl) continue;
+    const double c = std::ceil((double)n / cl_slots(t)) * cl_degree_us(A, P);
+    if (cluster == 0.0 || c < cluster) cluster = c;
+  }
+  if (cluster == 0.0) return false;
+  if (us) *us = std::min(step, cluster);
+  return g_cl_force > 0 || cluster < step;
 }
 
 template <class VT, int D>
@@ -1664,7 +1715,7 @@ int stencil_batch(int ncols, const evslcu_batch_col *cols, unsigned char *done) 
   if (g_cl_force >= 0)
     for (int c = 0; c < ncols; ++c) {
       const evslcu_batch_col &b = cols[c];
-      if (!stencil_ok(b.A) || b.deg < 1 || !cl_columns_pay(b.A, sizeof(double), ncols)) continue;
+      if (!stencil_ok(b.A) || b.deg < 1 || !cl_columns_pay(b.A, sizeof(double), 1)) continue;
       many.push_back(ClMany{b.A, b.mu, b.deg, b.cc, b.dd, b.x, b.y});
       done[c] = 1;
     }
