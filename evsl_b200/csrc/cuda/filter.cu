@@ -1,8 +1,9 @@
 // Chebyshev filter application y = p((A - cc)/dd) v (reference ChebAv,
 // SRC/chebpoly.c:519-598) and its dispatch.
 //
-// Default path: one fused kernel per degree (sparse.cu), launched with
-// programmatic dependent launch.  Optional path (evslx_set_filter_persistent):
+// Default paths: on a matrix with a merged stencil, one launch for all degrees
+// on a thread-block cluster or one per degree (stencil.cu); else one fused
+// kernel per degree (sparse.cu).  Launches use programmatic dependent launch.  Optional path (evslx_set_filter_persistent):
 // one cooperative launch for all degrees.  Every warp owns a fixed
 // set of SELL-32 chunks for the whole filter; each lane keeps, for each of
 // its rows, y and v_{k-1} in shared memory, so a degree step only streams A,
@@ -323,6 +324,7 @@ int evslcu_chebav(const evslcu_op *op, const double *mu, int deg, double cc, dou
   if (!op->A) return chebav_user_matvec(op, mu, deg, cc, dd, v, y, work, epi);
   const evslcu_mat *A = op->A;
   cudaEvent_t ev_a = nullptr;
+  const uint64_t launched_before = evslcu_launch_count();
   if (g_prof.on) {
     ev_a = prof_event();
     cudaEventRecord(ev_a, stream());
@@ -381,7 +383,10 @@ int evslcu_chebav(const evslcu_op *op, const double *mu, int deg, double cc, dou
   if (g_prof.on) {
     cudaEvent_t ev_b = prof_event();
     cudaEventRecord(ev_b, stream());
-    g_prof.pending.push_back({ev_a, ev_b, filter_bytes(A, deg, epi), deg});
+    // one launch per degree, or one for all of them (stencil.cu); a first call's
+    // timing of variants is not counted
+    const uint64_t launches = std::min<uint64_t>((uint64_t)deg, evslcu_launch_count() - launched_before);
+    g_prof.pending.push_back({ev_a, ev_b, filter_bytes(A, deg, epi), (int)launches});
   }
   return 0;
 }

@@ -1013,8 +1013,9 @@ int *cl_err() {
 
 template <class VT, int D, int CAP, bool ONE>
 int cl_max1() {
-  static int m = 0;
-  if (m) return m;
+  static int m = 0, dev = -1;  // limits are set per device
+  if (m && dev == lib_device()) return m;
+  dev = lib_device();
   if constexpr (CAP < 0)
     m = cl_limit((const void *)k_st_clusters<VT, D, ONE>, cl_threads(CAP, ONE));
   else
@@ -1188,7 +1189,9 @@ double cl_degree_us(const evslcu_mat *A, const ClPlan &P) {
 
 // Clusters of cl blocks that run at once (a block has an SM to itself).
 int cl_slots(int cl) {
-  static int slots[17] = {};
+  static int slots[17] = {}, dev = -1;
+  if (dev != lib_device()) std::fill(slots, slots + 17, 0);
+  dev = lib_device();
   if (slots[cl]) return slots[cl];
   cl_many_most(sizeof(double));  // sets the kernel's limits
   cudaLaunchConfig_t cfg = {};
@@ -1379,10 +1382,11 @@ int st_cols_group(const evslcu_mat *A, int nc, const ClMany *cols, VT *work) {
 template <int D>
 int kpm_cluster(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw,
                 bool *done) {
-  static int most = 0;  // most blocks per cluster, as cl_max1
-  const void *fn1 = (const void *)k_st_kpm_cluster<D, true>, *fn2 = (const void *)k_st_kpm_cluster<D, false>;
-  if (!most) {
+  static int most = 0, dev = -1;  // most blocks per cluster, as cl_max1
+  if (!most || dev != lib_device()) {
+    const void *fn1 = (const void *)k_st_kpm_cluster<D, true>, *fn2 = (const void *)k_st_kpm_cluster<D, false>;
     most = std::min(cl_limit(fn1, cl_threads(0, true)), cl_limit(fn2, cl_threads(0, false)));
+    dev = lib_device();
   }
   ClPlan P;
   for (int cl = 1; cl <= most; cl *= 2) {
@@ -1742,6 +1746,8 @@ void evslcu_stencil_release(void) {
   evslcu_free(g_cl_mu);
   g_cl_mu = nullptr;
   g_cl_mu_cap = 0;
+  if (g_cl_err) cudaFreeHost(g_cl_err);
+  g_cl_err = nullptr;
 }
 
 }  // extern "C"

@@ -400,7 +400,8 @@ int evslcu_set_pattern_const(int on);
  * variants on a matrix's first filter call and keeps the fastest; 0..6 forces
  * one (0/1 SELL-32 loop/unrolled, 2/3 pattern table in global memory
  * unrolled/loop, 4/5 pattern table in constant memory loop/unrolled, 6 the
- * constant table addressed by a per-row descriptor).  All give identical
+ * merged stencil, or without one the constant table addressed by a per-row
+ * descriptor).  All give identical
  * results. */
 int evslcu_set_cheb_variant(int v);
 /* At most this many blocks per degree step of the single-vector filter

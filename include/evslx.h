@@ -175,12 +175,16 @@ int evslx_row_pattern_count(void);
  * filter call on a matrix times each variant allowed for it and keeps the
  * fastest; 0..6 forces one: 0/1 SELL-32 with looped/unrolled row products,
  * 2/3 pattern table in global memory unrolled/looped, 4/5 pattern table in
- * constant memory looped/unrolled, 6 constant-memory table addressed by a
- * 4-byte descriptor per row, 7 the column-panel layout (2-6 need the
+ * constant memory looped/unrolled, 6 the merged stencil (a bit mask per row
+ * over one short list of entries) where the dictionary merges into one of at
+ * most 32 entries, else the constant-memory table addressed by a 4-byte
+ * descriptor per row, 7 the column-panel layout (2-6 need the
  * row-pattern dictionary, 4-6 its table in the constant pool, 7 the panel
  * layout; filtering fails with EVSLX_ERR_ARG when the forced variant is not
- * available).  Every variant gives the same result
- * bit for bit. */
+ * available).  With no variant forced, a matrix with a merged stencil runs on
+ * it (small ones in one launch for all degrees) without timing the others;
+ * asking for the times (evslx_filter_kernel) times them.  Every variant gives
+ * the same result bit for bit. */
 int evslx_set_filter_kernel(int variant);
 /* The registered matrix's chosen variant (-1: not chosen yet) and, when us is
  * not NULL, us[0..7] = measured microseconds per degree step of each variant
