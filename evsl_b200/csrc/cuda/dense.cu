@@ -20,6 +20,32 @@ namespace {
 constexpr double kEta = 0.70710678118654752440;  // 1/sqrt(2), SRC/misc_la.c:226
 constexpr int EVSL_NGS_MAX_CU = 2;                 // Gram-Schmidt passes, INC/internal_header.h:24
 
+// Launches of a Lanczos step come one after another with little work each:
+// with programmatic dependent launch the next grid is set up while this one
+// runs, and waits here until this one is complete.  ChebLanNr, 1,598 rows and
+// 20 pairs: 5.82 -> 5.13 ms; 9,797 rows and 241 pairs: 66.4 -> 64.2 ms.  A
+// grid that follows may start before the one ahead of this is complete, so it
+// loads nothing before its own wait that a recent launch wrote (a filter's
+// first degree loads masks only; its second starts after the first's wait).
+__device__ __forceinline__ void dependent_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int threads, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
 __global__ void k_dot(int n, const double *x, const double *y, double *part, unsigned int *ctr, double *out,
                       int sqrt_result) {
   __shared__ double sh[kThreads / 32];
@@ -50,6 +76,7 @@ __global__ void k_scal_inv_ds(int n, const double *s, double *x) {
 }
 
 __global__ void k_scal(int n, double a, double *x) {
+  dependent_start();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = __dmul_rn(a, x[i]);
 }
 
@@ -132,6 +159,7 @@ __device__ unsigned g_tile_ctr[kTileCtrs];
 __global__ void __launch_bounds__(kThreads)
     k_gemvT(int n, int k, const double *__restrict__ Q, long long ld, const double *__restrict__ v, double *part,
             int cols, int reduce, double alpha, double *h, const double *state) {
+  dependent_start();
   if (state && state[2] != 0.0) return;
   __shared__ double sv[kGemvTRows];
   __shared__ double sh[8][33];
@@ -244,6 +272,7 @@ __global__ void __launch_bounds__(kThreads)
     k_gemvN(int n, int k, const double *__restrict__ Q, long long ld, const double *__restrict__ h, double alpha,
             double *v, double *part, unsigned int *ctr, double *state, double *out, const double *d_alpha,
             double *host) {
+  dependent_start();
   if (state && state[2] != 0.0) return;
   __shared__ double sh_h[kGemvNChunk];
   __shared__ double sh[kThreads / 32];
@@ -278,7 +307,7 @@ int launch_gemvN(int n, int k, const double *Q, long long ld, const double *h, d
     case 2: fn = k_gemvN<2>; break;
     default: break;
   }
-  fn<<<g, kThreads, 0, stream()>>>(n, k, Q, ld, h, alpha, v, part, ctr, state, out, d_alpha, host);
+  EVSLCU_CUDA(launch_dependent(fn, dim3(g), kThreads, n, k, Q, ld, h, alpha, v, part, ctr, state, out, d_alpha, host));
   EVSLCU_LAUNCH_CHECK("k_gemvN");
   return 0;
 }
@@ -289,7 +318,8 @@ int launch_gemvT(int n, int k, const double *Q, long long ld, const double *v, d
   const int nchunks = (n + kGemvTRows - 1) / kGemvTRows;
   const int cols = gemvT_cols(nchunks, k), tiles = (k + cols - 1) / cols;
   const int reduce = tiles <= kTileCtrs ? 1 : 0;
-  k_gemvT<<<dim3(nchunks, tiles), kThreads, 0, stream()>>>(n, k, Q, ld, v, part, cols, reduce, alpha, h, state);
+  EVSLCU_CUDA(launch_dependent(k_gemvT, dim3(nchunks, tiles), kThreads, n, k, Q, ld, v, part, cols, reduce, alpha, h,
+                               state));
   EVSLCU_LAUNCH_CHECK("k_gemvT");
   if (!reduce) {
     k_gemvT_reduce<<<(k + 31) / 32, 256, 0, stream()>>>(nchunks, k, part, alpha, 0.0, h, state);
@@ -303,6 +333,7 @@ int launch_gemvT(int n, int k, const double *Q, long long ld, const double *v, d
 __global__ void __launch_bounds__(kThreads)
     k_cgs_start(int n, const double *coef, double sign, const double *x, double *y, double *part, unsigned int *ctr,
                 double *state) {
+  dependent_start();
   __shared__ double sh[kThreads / 32];
   const double c = x ? sign * (*coef) : 0.0;
   double s = 0.0;
@@ -890,7 +921,7 @@ int evslcu_scal_inv_ds(int n, const double *s_dev, double *x) {
 }
 
 int evslcu_scal(int n, double a, double *x) {
-  k_scal<<<grid_for(n), kThreads, 0, stream()>>>(n, a, x);
+  EVSLCU_CUDA(launch_dependent(k_scal, dim3(grid_for(n)), kThreads, n, a, x));
   EVSLCU_LAUNCH_CHECK("k_scal");
   return 0;
 }
@@ -1097,8 +1128,8 @@ static int cgs_pass(int n, int k, const double *Q, long long ldq, double *v, dou
 }
 
 static int cgs_start(int n, const double *coef, double sign, const double *x, double *v, double *state) {
-  k_cgs_start<<<grid_for(n, kThreads, 1024), kThreads, 0, stream()>>>(n, coef, sign, x, v, partials(),
-                                                                      counters() + CTR_NRM, state);
+  EVSLCU_CUDA(launch_dependent(k_cgs_start, dim3(grid_for(n, kThreads, 1024)), kThreads, n, coef, sign, x, v,
+                               partials(), counters() + CTR_NRM, state));
   EVSLCU_LAUNCH_CHECK("k_cgs_start");
   return 0;
 }
