@@ -347,6 +347,7 @@ def run_ours(args):
     kname = lib.FILTER_KERNELS[v_chosen] if v_chosen >= 0 else "sell-loop"
     if args.filter_kernel == "auto" and args.filter_mode == "per-degree" and lib.row_pattern_count() > 0:
         kname = "merged-stencil"  # grid operators run on their merged stencil; the variants are timed beside it
+        storage["filter_kernel"] = kname
     config1 = run_config1_ours(lib, lstream) if world == 1 else None
 
     # aggregate over ranks
@@ -408,9 +409,10 @@ def run_ours(args):
                 "frac_algorithmic": achieved / peak if peak else None,
                 "frac_dram": (traffic / avg_launch / 1e9 / peak) if (traffic and avg_launch and peak) else None,
                 "frac_note": "frac = frac_algorithmic: the formula's bytes (12 B per stored entry + vectors) over the "
-                             "kernel time; the row-pattern dictionary stores 2-byte ids and the per-degree working set "
-                             "stays in L2, so it exceeds 1; frac_dram = the DRAM bytes ncu measured per launch of this "
-                             "kernel variant (cold caches) over the same time",
+                             "kernel time; the operator is a byte or two per row (merged stencil or row-pattern "
+                             "dictionary) and the vectors stay in L2, so it exceeds 1 and is no share of what HBM "
+                             "moved; frac_dram = the DRAM bytes ncu measured per launch of this kernel variant with "
+                             "cold caches over the same time, an upper figure: in the solve most come from L2",
                 "traffic": traffic,
                 "traffic_kernel": "k_cheb:" + kname,
                 "algorithmic_bytes_per_launch": f_bytes / f_launch if f_launch else None,

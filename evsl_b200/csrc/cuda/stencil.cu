@@ -17,6 +17,9 @@
 //     thousand rows 4.57 -> 3.15, 10^4 rows 2.95 -> 2.4 (launch latency).
 //   * k_st_cluster: every degree in one launch, for operators whose vectors
 //     fit the shared memory of one thread-block cluster: 10^4 rows 2.4 -> 0.52.
+//   * k_st_cols, k_st_clusters: the same two for several columns, each with
+//     its own polynomial; k_st_kpm, k_st_kpm_cluster: the same two with the
+//     KPM recurrence's inner products; k_st_spmv: the plain product.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
