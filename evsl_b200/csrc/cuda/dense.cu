@@ -25,8 +25,8 @@ constexpr int EVSL_NGS_MAX_CU = 2;                 // Gram-Schmidt passes, INC/i
 // runs, and waits here until this one is complete.  ChebLanNr, 1,598 rows and
 // 20 pairs: 5.82 -> 5.13 ms; 9,797 rows and 241 pairs: 66.4 -> 64.2 ms.  A
 // grid that follows may start before the one ahead of this is complete, so it
-// loads nothing before its own wait that a recent launch wrote (a filter's
-// first degree loads masks only; its second starts after the first's wait).
+// loads nothing before its own wait that a launch wrote which the host has not
+// waited for (a filter's degrees load masks only).
 __device__ __forceinline__ void dependent_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -13,8 +13,8 @@
 //     term), and adding them one after another is the same sum in the same
 //     order at 16 / 3 instead of 16 bytes of y per row and degree.
 //     Against the dictionary kernels before it (sparse.cu, the fastest of the
-//     seven timed): 3-D Laplacian of 10^6 rows 7.84 -> 6.30 us a degree, 343
-//     thousand rows 4.57 -> 3.15, 10^4 rows 2.95 -> 2.4 (launch latency).
+//     seven timed): 3-D Laplacian of 10^6 rows 7.84 -> 6.49 us a degree, 343
+//     thousand rows 4.57 -> 3.56, 10^4 rows 2.95 -> 2.4 (launch latency).
 //   * k_st_cluster: every degree in one launch, for operators whose vectors
 //     fit the shared memory of one thread-block cluster: 10^4 rows 2.4 -> 0.52.
 //   * k_st_cols, k_st_clusters: the same two for several columns, each with
@@ -64,7 +64,8 @@ struct StY {
 // Returns the sum of dotv[r] y[r] over the thread's rows (EPI).  yd: where the
 // finished y goes (the last degree), else null.
 // each(x, w) is called for every row, with its values of v_k and of the result.
-template <class VT, int D, int J, bool FIRST, bool EPI, class F>
+// OWN (J > 1): a row's own v_k is loaded before the masks are looked at.
+template <class VT, int D, int J, bool FIRST, bool EPI, bool OWN, class F>
 __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &M, const VT *__restrict__ vk,
                                           const VT *vkm1, VT *out, VT *y, double *yd, VT t, VT ncc, const StY<VT> &Y,
                                           const double *__restrict__ zold, double nbeta,
@@ -80,11 +81,15 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
     }
     r0 = c < M.cols ? (int)q * J * M.S + rem : A.n;
   }
-  // The masks never change, and v_k-1 was written two launches ago: that one
-  // has completed once the previous launch has let this one start (it does so
-  // after its own wait).
+  // Only the masks are loaded before the wait: the host has waited for the
+  // kernel that wrote them (stencil_build).  v_k-1 was written two launches
+  // ago, but it is the wait that makes other launches' writes visible.  (Loaded
+  // before it, v_k-1 overlapped the launch ahead: 3.15 instead of 3.56 us a
+  // degree on 343 thousand rows, 6.30 instead of 6.49 on 10^6.)  What needs no
+  // mask is loaded before the masks are looked at, which costs the blocks that
+  // start after the wait no second latency: 10^6 rows 6.87 -> 6.49; OWN gains in
+  // one column's launches and loses where many columns fill the chip.
   unsigned m[J];
-  VT xm1[J];
   bool live[J];
   bool all = true;
 #pragma unroll
@@ -92,17 +97,23 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
     const int r = r0 + j * M.S;
     live[j] = r < A.n;
     m[j] = live[j] ? (unsigned)__ldg(A.mask + r) : 0u;
-    xm1[j] = (!FIRST && live[j]) ? vkm1[r] : (VT)0;
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const VT *xr = vk + r0;
+  VT acc[J], x[J], xm1[J], yo[J];
+#pragma unroll
+  for (int j = 0; j < J; ++j) xm1[j] = (!FIRST && live[j]) ? vkm1[r0 + j * M.S] : (VT)0;
+#pragma unroll
+  for (int j = 0; j < J; ++j) yo[j] = (Y.terms && !Y.init && live[j]) ? y[r0 + j * M.S] : (VT)0;
+  VT own[J];  // OWN
+  if (OWN) {
+#pragma unroll
+    for (int j = 0; j < J; ++j) own[j] = live[j] ? __ldg(xr + j * M.S) : (VT)0;
   }
 #pragma unroll
   for (int j = 0; j < J; ++j) all = all && m[j] == A.full;
   all = __all_sync(0xffffffffu, all);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const VT *xr = vk + r0;
-  VT acc[J], x[J], yo[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) yo[j] = (Y.terms && !Y.init && live[j]) ? y[r0 + j * M.S] : (VT)0;
   if constexpr (J == 1) {
     acc[0] = (VT)0;
     x[0] = (VT)0;
@@ -127,7 +138,7 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
     VT p[J + 2], g[J][D];
     if (all) {
 #pragma unroll
-      for (int j = 0; j < J + 2; ++j) p[j] = __ldg(xr + (j - 1) * M.S);
+      for (int j = 0; j < J + 2; ++j) p[j] = (OWN && j >= 1 && j <= J) ? own[j - 1] : __ldg(xr + (j - 1) * M.S);
 #pragma unroll
       for (int j = 0; j < J; ++j)
 #pragma unroll
@@ -145,7 +156,7 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
 #pragma unroll
       for (int j = 0; j < J + 2; ++j) {
         const bool have = j == 0 ? (m[0] & 1u) != 0 : j == J + 1 ? (m[J - 1] >> (D - 1) & 1u) != 0 : live[j == 0 ? 0 : j > J ? J - 1 : j - 1];
-        p[j] = have ? __ldg(xr + (j - 1) * M.S) : (VT)0;
+        p[j] = (OWN && j >= 1 && j <= J) ? own[j - 1] : have ? __ldg(xr + (j - 1) * M.S) : (VT)0;
       }
 #pragma unroll
       for (int j = 0; j < J; ++j)
@@ -202,8 +213,8 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
               const double *__restrict__ zold, double nbeta, const double *__restrict__ dotv, double *part,
               unsigned int *ctr, double *dot_out) {
   __shared__ double sh[EPI ? kThreads / 32 : 1];
-  const double dsum = st_rows<double, D, J, FIRST, EPI>(A, M, vk, vkm1, out, y, yd, t, ncc, Y, zold, nbeta, dotv,
-                                                        [](double, double) {});
+  const double dsum = st_rows<double, D, J, FIRST, EPI, J == 2>(A, M, vk, vkm1, out, y, yd, t, ncc, Y, zold, nbeta,
+                                                                dotv, [](double, double) {});
   if (EPI && dot_out) {
     const double b = block_sum(dsum, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = b;
@@ -246,8 +257,8 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
     Y.c1 = (VT)__ldg(I.mu + k - 1);
     Y.c2 = (VT)__ldg(I.mu + (FIRST ? 0 : k - 2));
   }
-  st_rows<VT, D, J, FIRST, false>(A, M, I.vk, I.vkm1, I.out, I.y, I.yd, I.t, I.ncc, Y, nullptr, 0.0, nullptr,
-                                  [](VT, VT) {});
+  st_rows<VT, D, J, FIRST, false, false>(A, M, I.vk, I.vkm1, I.out, I.y, I.yd, I.t, I.ncc, Y, nullptr, 0.0, nullptr,
+                                         [](VT, VT) {});
 }
 
 // One KPM step (two moments per product, as k_kpm_dbl in sparse.cu) for the
@@ -264,12 +275,12 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
   const long long at = (long long)blockIdx.y * A.n;
   double s[3] = {0.0, 0.0, 0.0};
   const StY<double> Y{0, 0, 0.0, 0.0, 0.0};
-  st_rows<double, D, J, FIRST, false>(A, M, vk + at, FIRST ? nullptr : vkm1 + at, out + at, nullptr, nullptr, t, ncc,
-                                      Y, nullptr, 0.0, nullptr, [&](double x, double w) {
-                                        s[0] += w * w;
-                                        s[1] += w * x;
-                                        if (FIRST) s[2] += x * x;
-                                      });
+  st_rows<double, D, J, FIRST, false, false>(A, M, vk + at, FIRST ? nullptr : vkm1 + at, out + at, nullptr, nullptr, t,
+                                             ncc, Y, nullptr, 0.0, nullptr, [&](double x, double w) {
+                                               s[0] += w * w;
+                                               s[1] += w * x;
+                                               if (FIRST) s[2] += x * x;
+                                             });
   // one barrier for all the sums (block_sum's two each kept the warps of a
   // block waiting a third of the time)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -328,15 +339,17 @@ __global__ void k_st_float(int n, const double *__restrict__ x, float *out) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) out[r] = (float)x[r];
 }
 
-// Two rows per thread where the grid still covers every SM's warps about
-// once.  Measured, us a degree, 1 / 2 / 3 rows per thread: 125 thousand rows
-// 2.58 / 2.57 / 2.77, 343 thousand 3.21 / 3.15 / 3.47, 10^6 (3-D) 6.51 / 6.30 /
-// 6.82, 10^6 (2-D) 5.45 / 5.28 / 5.47, 4.1 million 29.1 / 25.5 / 26.3.
+// Two rows per thread: several columns from kStTwoRows rows on; one column where
+// one row per thread would need more blocks than run at once (6 on an SM).
+// Measured, us a degree of one column, 1 / 2 rows per thread: 215 thousand rows
+// 2.73 / 3.41, 343 thousand 3.57 / 3.56, 450 thousand 3.81 / 4.17, 592 thousand
+// 4.50 / 4.59, 10^6 (3-D) 6.35 / 6.49, 10^6 (2-D) 5.74 / 5.37, 4.1 million
+// 25.3 / 25.3; three rows were 4-8% slower than two at every size.
 constexpr int kStTwoRows = 150000;
 
-StMarch st_march(int n, int span, bool sym) {
+StMarch st_march(int n, int span, bool sym, bool one_column) {
   StMarch M;
-  int J = n >= kStTwoRows ? 2 : 1;
+  int J = (one_column ? n > 6 * kThreads * sm_count() : n >= kStTwoRows) ? 2 : 1;
   if (!sym || span < 1 || (long long)span * J > n || n > (1 << 29)) J = 1;
   M.S = J > 1 ? span : std::max(n, 1);
   M.J = J;
@@ -350,7 +363,7 @@ template <int D>
 int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y, double t,
             double ncc, const StY<double> &Y, bool last, const evslcu_cheb_epi *ep) {
   const StArg<double, D> S = st_arg<double, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], true);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads);
   cfg.blockDim = dim3(kThreads);
@@ -1295,7 +1308,7 @@ bool cl_columns_pay(const evslcu_mat *A, size_t vb, int n, double *us = nullptr)
 template <class VT, int D>
 int st_cols_launch(const evslcu_mat *A, int na, const StStepCols<VT> &C, int k) {
   const StArg<VT, D> S = st_arg<VT, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], false);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads, na);
   cfg.blockDim = dim3(kThreads);
@@ -1435,7 +1448,7 @@ int kpm_cluster(const evslcu_mat *A, int steps, int nvec, const double *probes, 
 template <int D>
 int kpm_steps(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw) {
   const StArg<double, D> S = st_arg<double, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1]);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], false);
   const size_t n = (size_t)A->n;
   const int grid = (M.cols + kThreads - 1) / kThreads;
   const int group = (int)std::max<size_t>(1, std::min<size_t>((size_t)nvec, kStColsBytes / (16 * n)));
@@ -1566,6 +1579,8 @@ int stencil_build(evslcu_mat *M) {
     }
     count_launch();
     rc = check_launch("k_st_mask");
+    // the filter kernels read the masks before they wait for the launch ahead
+    if (!rc) rc = evslcu_sync();
   }
   evslcu_free(tab);
   if (rc) {

@@ -63,7 +63,13 @@ SHAPES = {
     "two-rows-7": (160003, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
     "two-rows-dropped": (151000, [(-900, -1.0), (-30, 0.2), (-1, -1.0), (0, 6.0), (1, -1.0), (30, 0.2), (900, -1.0)], 7),
     "two-rows-9": (155555, box9(400), 0),
+    # one column's threads take two rows from one wave of blocks on (227,328 rows)
+    "one-wave-7": (227328, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
+    "over-one-wave-7": (227329, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
+    "over-one-wave-5-dropped": (231001, [(-487, -1.0), (-1, 0.3), (0, 4.0), (1, 0.3), (487, -1.0)], 5),
+    "over-one-wave-9": (230400, box9(480), 0),
     # the march's stride is more than half the rows: one row per thread again
+    "wide-offset-one-column": (230001, [(-120000, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (120000, -1.0)], 0),
     "wide-offset": (150100, [(-80000, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (80000, -1.0)], 0),
 }
 
@@ -205,3 +211,27 @@ def test_kpm_on_stencils(gpu_lib, shape, blocks):
     finally:
         gpu_lib.set_row_patterns(True)
         gpu_lib.lib.evslcu_set_stencil_cluster(0)
+
+
+@pytest.mark.parametrize("shape", ["over-one-wave-7", "cluster-over"])
+def test_filter_right_after_registration_on_the_device(gpu_lib, shape):
+    """SetAMatrix_device_csr, then ChebAv on device vectors with nothing in
+    between: the filter's first loads see the masks of the matrix just
+    registered, not of the one before it (the pool gives both the same
+    memory)."""
+    n, entries, _ = SHAPES[shape]
+    lib = gpu_lib.lib
+    bound = sum(abs(v) for _, v in entries)
+    pol, mu = polynomial(gpu_lib, 5, bound)
+    v = O.seeded_normal(n, 3)
+    dv, dy, dw = (E.DeviceBuffer.from_host(lib, a) for a in (v, v, np.zeros(3 * n)))
+    full, thin = stencil_csr(n, entries), stencil_csr(n, entries, 3)
+    refs = [O.cheb_av(pol.as_dict(), *m, v) for m in (full, thin)]
+    try:
+        lib.evslcu_set_stencil_cluster(-1)
+        for i in range(12):
+            gpu_lib.set_csr_device(*((full, thin)[i % 2]))
+            assert lib.ChebAv(C.byref(pol), dv.ptr, dy.ptr, dw.ptr) == 0
+            assert np.array_equal(dy.to_host(), refs[i % 2]), i
+    finally:
+        lib.evslcu_set_stencil_cluster(0)
