@@ -308,6 +308,7 @@ int evslcu_set_wait_limit(unsigned long long polls) {
   g_barrier_polls = polls ? polls : kBarrierSpinLimit;
   set_wave_wait_limit(polls);
   set_batch_wait_limit(polls);
+  set_cluster_wait_limit(polls);
   return 0;
 }
 

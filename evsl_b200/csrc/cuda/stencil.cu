@@ -491,24 +491,37 @@ __device__ __forceinline__ void bar_expect(unsigned long long *bar, unsigned byt
                "r"(bytes)
                : "memory");
 }
-// Waits for the phase of the given parity; false when the polls run out, or at
-// once when another wait of the block has.
+// Waits for the phase of the given parity; false when the polls run out, or
+// after one poll when another wait of the block has.  The first poll returns at
+// once, each later one suspends the thread for up to a microsecond, so that the
+// default limit is about a second.
 constexpr int kClPolls = 1 << 20;
+int g_cl_polls = kClPolls;
 __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity, int polls, const int *dead) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-  for (int i = 0; i < polls; ++i) {
-    unsigned ok;
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(a), "r"(parity)
+      : "memory");
+  for (int i = 1; !ok && i < polls && !*(const volatile int *)dead; ++i)
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(a), "r"(parity)
+        : "r"(a), "r"(parity), "r"(1000)
         : "memory");
-    if (ok) return true;
-    if (*(const volatile int *)dead) break;
-  }
-  return false;
+  return ok != 0;
+}
+// The end of a block that gave up, after a cluster barrier that the others
+// reach (or leave the kernel) without sending again: values already on their
+// way to its shared memory need a microsecond or two to arrive.
+__device__ __forceinline__ void linger() {
+  for (int i = 0; i < 100; ++i) __nanosleep(1000);
 }
 
 // Shared memory: two vectors of R rows with a halo on both sides, which take
@@ -530,9 +543,15 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
 // after a degree's rows, in place of the stores as they are computed, was 3-10%
 // slower at every halo width.)
 //
-// A wait that runs out of polls sets *err (the host's mapped flag) and `dead`:
-// later waits of the block give up at once, and it stays until the blocks that
-// may still send to it are done.
+// A wait that runs out of polls sets *err (the host's mapped flag) and `dead`.
+// From the next degree on the block announces no bytes, sends none and waits no
+// more; it goes through its remaining degrees with whatever is there.  Its
+// neighbours run out of polls in turn, at most two degrees later, so at most
+// two degrees' bytes reach an mbarrier that does not expect them (its count
+// takes 2^20 - 1).  The block's threads agree on `dead` at a barrier after the
+// last degree, and a block that gave up stays until every other has left its
+// last degree, at one cluster barrier; where the epilogue's sum has a cluster
+// barrier for all blocks, it is that one.
 //
 // MANY: the launch's blocks may have more threads than this column's rows need
 // (R is a multiple of a warp, so whole warps sit out).
@@ -621,13 +640,15 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
       c1 = (VT)mu(k - 1);
       c2 = (VT)mu(FIRST ? 0 : k - 2);
     }
-    if (!LAST && tid == 0 && expect && !*(volatile int *)&dead) bar_expect(bars + (k & 1), expect);
+    bool stop = !FIRST && *(volatile int *)&dead;
+    if (!LAST && tid == 0 && expect && !stop) bar_expect(bars + (k & 1), expect);
     if (!FIRST && edge && !bar_wait(bars + ((k - 1) & 1), (unsigned)((k - 2) >> 1) & 1u, polls, &dead)) {
+      stop = true;
       *(volatile int *)&dead = 1;
       *(volatile int *)err = 1;
     }
     const unsigned bk = (unsigned)((k & 1) * 8);
-    unsigned fb = fast, eb = edge;
+    unsigned fb = fast, eb = stop ? 0u : edge;  // eb: iterations that send
 #pragma unroll 2
     for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T, fb >>= 1, eb >>= 1) {
       if (MANY && i >= R) continue;
@@ -726,7 +747,11 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
     }
     degree(k, no, yes, yes);
   }
-  if (cl > 1 && dead) cluster_sync();  // nobody's memory goes away while others may still send to it
+  bool gave_up = false;
+  if (cl > 1) {
+    __syncthreads();
+    gave_up = dead != 0;
+  }
   if (I.dot_out) {
     // the blocks' sums in rank order, added by block 0
     const double b = block_sum(dsum, red);
@@ -741,7 +766,10 @@ __device__ __forceinline__ void st_cluster_body(const StCol &I, MU mu, int polls
     } else if (tid == 0) {
       *I.dot_out = b;
     }
+  } else if (gave_up) {
+    cluster_sync();
   }
+  if (gave_up) linger();
 }
 
 // One cluster filters `one`, whose coefficients (up to CAP) come with the
@@ -855,14 +883,16 @@ __global__ void __launch_bounds__(cl_threads(0, ONE), 1)
     constexpr bool FIRST = decltype(first_c)::value;
     const bool last = k == steps;
     const double t = FIRST ? I.t1 : I.t2;
-    if (!last && tid == 0 && expect && !*(volatile int *)&dead) bar_expect(bars + (k & 1), expect);
+    bool stop = !FIRST && *(volatile int *)&dead;
+    if (!last && tid == 0 && expect && !stop) bar_expect(bars + (k & 1), expect);
     if (!FIRST && edge && !bar_wait(bars + ((k - 1) & 1), (unsigned)((k - 2) >> 1) & 1u, polls, &dead)) {
+      stop = true;
       *(volatile int *)&dead = 1;
       *(volatile int *)err = 1;
     }
     const unsigned bk = (unsigned)((k & 1) * 8);
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    unsigned fb = fast, eb = edge;
+    unsigned fb = fast, eb = stop ? 0u : edge;  // eb: iterations that send
     for (int it = 0, i = tid + (nit - 1) * T; it < nit; ++it, i = it == 1 ? tid : i + T, fb >>= 1, eb >>= 1) {
       const double *xs = src + i;
       double acc = 0.0, x, xm1 = 0.0, g[D];
@@ -932,7 +962,10 @@ __global__ void __launch_bounds__(cl_threads(0, ONE), 1)
   };
   step(1, std::true_type{});
   for (int k = 2; k <= steps; ++k) step(k, std::false_type{});
-  if (cl > 1 && dead) cluster_sync();  // nobody's memory goes away while others may still send to it
+  if (cl > 1 && dead) {  // as st_cluster_body; the last step ended with a barrier
+    cluster_sync();
+    linger();
+  }
 }
 
 // raw[i] = part[i * cl] + part[i * cl + 1] + ...
@@ -1061,8 +1094,8 @@ int cl_launch(const StCol &one, const double *mu, const ClPlan &P) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, true>, one, mus, kClPolls, err)
-                           : cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, false>, one, mus, kClPolls, err);
+  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, true>, one, mus, g_cl_polls, err)
+                           : cudaLaunchKernelEx(&cfg, k_st_cluster<VT, D, CAP, false>, one, mus, g_cl_polls, err);
   if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "cluster filter launch failed: %s", cudaGetErrorString(e));
   EVSLCU_LAUNCH_CHECK("k_st_cluster");
   return 0;
@@ -1096,8 +1129,8 @@ int cl_launch_many(int ncols, const StTab &tab, int cl, int T, size_t smem, bool
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = one ? cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, true>, tab, kClPolls, err)
-                      : cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, false>, tab, kClPolls, err);
+  cudaError_t e = one ? cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, true>, tab, g_cl_polls, err)
+                      : cudaLaunchKernelEx(&cfg, k_st_clusters<VT, D, false>, tab, g_cl_polls, err);
   if (e != cudaSuccess) return fail(EVSLCU_ERR_CUDA, "cluster filter launch failed: %s", cudaGetErrorString(e));
   EVSLCU_LAUNCH_CHECK("k_st_clusters");
   return 0;
@@ -1429,8 +1462,8 @@ int kpm_cluster(const evslcu_mat *A, int steps, int nvec, const double *probes, 
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, true>, C, part, nvec, kClPolls, err)
-                             : cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, false>, C, part, nvec, kClPolls, err);
+  cudaError_t e = P.R == P.T ? cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, true>, C, part, nvec, g_cl_polls, err)
+                             : cudaLaunchKernelEx(&cfg, k_st_kpm_cluster<D, false>, C, part, nvec, g_cl_polls, err);
   int rc = e == cudaSuccess ? 0 : fail(EVSLCU_ERR_CUDA, "KPM cluster launch failed: %s", cudaGetErrorString(e));
   count_launch();
   if (!rc) rc = check_launch("k_st_kpm_cluster");
@@ -1618,6 +1651,10 @@ int stencil_error() {
   if (!g_cl_err || !*(volatile int *)g_cl_err) return 0;
   *(volatile int *)g_cl_err = 0;
   return fail(EVSLCU_ERR_TIMEOUT, "a wait of the filter kernel did not complete within its bound");
+}
+
+void set_cluster_wait_limit(unsigned long long polls) {
+  g_cl_polls = (polls == 0 || polls > (unsigned long long)kClPolls) ? kClPolls : (int)polls;
 }
 
 bool stencil_ok(const evslcu_mat *M) { return M->st_d > 0 && M->use_pat && M->kernel == 0; }

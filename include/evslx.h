@@ -147,8 +147,12 @@ int evslx_matrix_sell_layout(int *sigma, long long *stored, long long *stored_un
 int evslx_set_filter_wave(int on);
 /* Every device-side wait is bounded: a block of the single-launch filter
  * gives up at a grid barrier after 2^26 polls (about 2 s), a tile of the
- * pipelined filter after 2^22 polls on a dependency; the call then returns
- * EVSLX_ERR_TIMEOUT and the library stays usable.  This sets both limits
+ * pipelined filter and a column of the persistent batch after 2^22 polls on a
+ * dependency, a block of a cluster filter (small matrices with a merged
+ * stencil, their KPM moments included) after 2^20 polls of about a microsecond
+ * on its neighbours' rows; the call then returns EVSLX_ERR_TIMEOUT, or the
+ * next one that waits for the device where the call itself does not, and the
+ * library stays usable.  This sets all limits
  * (0 restores the defaults); a very small limit makes the waits run out,
  * which tests of the failure path use. */
 int evslx_set_wait_limit(unsigned long long polls);

@@ -235,3 +235,56 @@ def test_filter_right_after_registration_on_the_device(gpu_lib, shape):
             assert np.array_equal(dy.to_host(), refs[i % 2]), i
     finally:
         lib.evslcu_set_stencil_cluster(0)
+
+
+@pytest.mark.parametrize("call", ["filter", "lanczos", "columns", "columns-fp32", "kpm", "engine"])
+def test_cluster_waits_run_out_and_library_recovers(gpu_lib, call):
+    """With a limit of one poll the blocks of the cluster kernels give up on
+    their neighbours' rows: the call returns EVSLX_ERR_TIMEOUT (-105) with every
+    block gone, and with the default limit the same call gives its result of
+    before, bit for bit."""
+    ia, ja, a = O.lap_csr(101, 97, 1)
+    n = len(ia) - 1
+    gpu_lib.set_csr(ia, ja, a)
+    X = O.seeded_normal(4 * n, 8).reshape(4, n)
+    iv = [0.5, 0.6, 0.0, 8.0]
+    pol = gpu_lib.find_pol(iv)
+    mat = gpu_lib.matrix(ia, ja, a)
+    dX = E.DeviceBuffer.from_host(gpu_lib.lib, X)
+
+    def engine():
+        eng = gpu_lib.engine(1, precision=E.PREC_FP64)
+        try:
+            eng.submit_slice(mat, iv, pol, 400, 1e-8, X[0], 1)
+            eng.run()
+            return eng.pop()["lam"]
+        finally:
+            eng.free()
+
+    run = {
+        "filter": lambda: gpu_lib.chebav(pol, X[0]),
+        "lanczos": lambda: gpu_lib.cheblan_nr(iv, 400, 1e-8, X[0], pol)[0],
+        "columns": lambda: gpu_lib.chebav_multi([pol] * 4, X, E.PREC_FP64),
+        "columns-fp32": lambda: gpu_lib.chebav_multi([pol] * 4, X, E.PREC_MIXED),
+        "kpm": lambda: gpu_lib.kpm_dots(60, iv, dX, 4),
+        "engine": engine,
+    }[call]
+    try:
+        ref = run()
+        assert len(ref) > 0 and np.all(np.isfinite(ref))
+        gpu_lib.set_wait_limit(1)
+        codes = []
+        for _ in range(3):
+            try:
+                run()
+                codes.append(0)
+            except E.EvslError as e:
+                codes.append(-105 if "returned -105" in str(e) else str(e))
+                assert "within its bound" in gpu_lib.last_error()
+        assert -105 in codes and all(c in (0, -105) for c in codes), codes
+        gpu_lib.set_wait_limit(0)
+        assert np.array_equal(run(), ref)
+    finally:
+        gpu_lib.set_wait_limit(0)
+        mat.free()
+        gpu_lib.free_pol(pol)
