@@ -1012,7 +1012,7 @@ int evslcu_filter_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu
   if (rc) return rc;
   if (!work || work_bytes < evslcu_filter_columns_work(A->n, fp32, ncols))
     return fail(EVSLCU_ERR_ARG, "filter_columns: work too small");
-  if (g_mf_variant < 0 && stencil_columns_ok(A, ncols, cols)) {
+  if (g_mf_variant < 0 && stencil_columns_ok(A, fp32, ncols, cols, true)) {
     std::vector<size_t> off((size_t)ncols);
     double *mu = stencil_columns_mu(ncols, cols, off.data(), &rc);
     if (!rc) rc = stencil_columns(A, fp32, ncols, cols, mu, off.data(), work);
@@ -1058,7 +1058,7 @@ evslcu_filter_plan *evslcu_filter_plan_create(const evslcu_mat *A, int fp32, int
     evslcu_filter_plan_destroy(P);
     return nullptr;
   }
-  if (g_mf_variant < 0 && stencil_columns_ok(A, ncols, cols)) {
+  if (g_mf_variant < 0 && stencil_columns_ok(A, fp32, ncols, cols, false)) {
     int err = 0;
     P->st_cols = (evslcu_filter_col *)malloc(sizeof(evslcu_filter_col) * (size_t)ncols);
     P->st_off = (size_t *)malloc(sizeof(size_t) * (size_t)ncols);
@@ -1110,6 +1110,8 @@ int evslcu_filter_plan_run(evslcu_filter_plan *P, const double *const *x, double
       P->st_cols[c].x = x[c];
       P->st_cols[c].y = y[c];
     }
+    if (!stencil_columns_ok(P->A, P->fp32, P->ncols, P->st_cols, true))
+      return evslcu_filter_columns(P->A, P->fp32, P->ncols, P->st_cols, P->work, P->work_bytes);
     return stencil_columns(P->A, P->fp32, P->ncols, P->st_cols, P->st_mu, P->st_off, P->work);
   }
   for (int c = 0; c < P->ncols; ++c) {

@@ -490,7 +490,7 @@ int chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, double cc
 int stencil_build(evslcu_mat *M);
 void stencil_free(evslcu_mat *M);
 bool stencil_ok(const evslcu_mat *M);
-bool stencil_columns_ok(const evslcu_mat *A, int ncols, const evslcu_filter_col *cols);
+bool stencil_columns_ok(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, bool vectors);
 double *stencil_columns_mu(int ncols, const evslcu_filter_col *cols, size_t *off, int *err);
 int stencil_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, const double *dmu,
                     const size_t *off, void *work);

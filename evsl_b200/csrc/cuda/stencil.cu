@@ -1707,13 +1707,32 @@ int stencil_kpm(const evslcu_mat *A, int steps, int nvec, const double *probes, 
   }
 }
 
+// Whether every column's y may be written while other columns' x are read:
+// y's share no memory with x's, except that a column may be filtered in place.
+// (One FP64 launch per degree reads x at degrees 1 and 2, a row's own value
+// last, and writes y from degree 2 on, or at degree 1 when that is all; the
+// other kernels copy x first.)
+static bool columns_apart(int n, int fp32, int ncols, const evslcu_filter_col *cols) {
+  std::vector<std::pair<uintptr_t, int>> y((size_t)ncols);
+  for (int c = 0; c < ncols; ++c) y[c] = {(uintptr_t)cols[c].y, c};
+  std::sort(y.begin(), y.end());
+  const uintptr_t bytes = sizeof(double) * (uintptr_t)n;
+  for (int c = 0; c < ncols; ++c) {
+    const uintptr_t x = (uintptr_t)cols[c].x;
+    auto it = std::upper_bound(y.begin(), y.end(), std::make_pair(x > bytes ? x - bytes : 0, ncols));
+    for (; it != y.end() && it->first < x + bytes; ++it)
+      if (it->first != x || it->second != c || (!fp32 && cols[c].deg == 1)) return false;
+  }
+  return true;
+}
+
 // Whether filter_columns takes these columns: a merged stencil, every degree
-// at least 1.
-bool stencil_columns_ok(const evslcu_mat *A, int ncols, const evslcu_filter_col *cols) {
+// at least 1, and (once the vectors are known) no y in another column's way.
+bool stencil_columns_ok(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, bool vectors) {
   if (!stencil_ok(A)) return false;
   for (int c = 0; c < ncols; ++c)
     if (cols[c].deg < 1) return false;
-  return true;
+  return !vectors || columns_apart(A->n, fp32, ncols, cols);
 }
 
 // Device copy of the columns' coefficients, one after another (columns that

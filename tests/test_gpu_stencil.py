@@ -288,3 +288,27 @@ def test_cluster_waits_run_out_and_library_recovers(gpu_lib, call):
         gpu_lib.set_wait_limit(0)
         mat.free()
         gpu_lib.free_pol(pol)
+
+
+@pytest.mark.parametrize("blocks", [-1, 0])
+@pytest.mark.parametrize("prec", [E.PREC_FP64, E.PREC_MIXED])
+@pytest.mark.parametrize("shape", ["cluster-over", "two-rows-7"])
+@pytest.mark.parametrize("shift", [0, 1, -1])
+def test_columns_in_place(gpu_lib, shift, shape, prec, blocks):
+    """Y on X itself, and each column's result on its neighbour's vector: the
+    columns of separate vectors, degree 1 included."""
+    n, entries, _ = SHAPES[shape]
+    lib = gpu_lib.lib
+    gpu_lib.set_csr(*stencil_csr(n, entries))
+    bound = sum(abs(v) for _, v in entries)
+    made = [polynomial(gpu_lib, deg, bound) for deg in (1, 2, 3, 1, 5)]
+    pols = (E.PolParams * 5)(*[p for p, _ in made])
+    X = O.seeded_normal(7 * n, 4).reshape(7, n)
+    try:
+        lib.evslcu_set_stencil_cluster(blocks)
+        ref = gpu_lib.chebav_multi([p for p, _ in made], X[1:6], prec)
+        buf = E.DeviceBuffer.from_host(lib, X)
+        assert lib.evslx_chebav_multi(5, pols, buf.ptr + 8 * n, buf.ptr + 8 * n * (1 + shift), prec) == 0
+        assert np.array_equal(buf.to_host(shape=X.shape)[1 + shift:6 + shift], ref)
+    finally:
+        lib.evslcu_set_stencil_cluster(0)
