@@ -221,8 +221,19 @@ int evslcu_last_cuda_error(char *buf, int len) {
   return e == cudaSuccess ? 0 : EVSLCU_ERR_CUDA;
 }
 
+static size_t g_malloc_limit = 0;
+
+int evslcu_set_malloc_limit(size_t nbytes) {
+  g_malloc_limit = nbytes;
+  return 0;
+}
+
 void *evslcu_malloc(size_t nbytes) {
   void *p = nullptr;
+  if (g_malloc_limit && nbytes > g_malloc_limit) {
+    fail(EVSLCU_ERR_NOMEM, "allocation of %zu bytes is above the limit set for tests", nbytes);
+    return nullptr;
+  }
   if (nbytes == 0) nbytes = 1;
   cudaError_t e = pool_ready() ? cudaMallocFromPoolAsync(&p, nbytes, g_pool, g_ctx.stream) : cudaMalloc(&p, nbytes);
   if (e == cudaErrorMemoryAllocation && pool_ready()) {

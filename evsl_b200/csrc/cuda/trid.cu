@@ -72,8 +72,8 @@ __global__ void __launch_bounds__(kTridThreads)
   if (lane == 0) w[i] = 0.5 * (lo + hi);
 }
 
-// Inverse iteration for eigenvectors j0 .. j0 + m - 1 of T (shift j in
-// shift[j]): one thread per vector, the arithmetic of the host's
+// Inverse iteration for eigenvectors num[0] .. num[m - 1] of T at shift[0] ..
+// shift[m - 1], into the columns num[] of Z: one thread per vector, the arithmetic of the host's
 // (invit_range, host/tridiag.c) operation for operation, so the vectors are
 // the same bit for bit.  A vector is a chain of a few thousand dependent
 // divisions and updates that costs the host 60 us at 850 rows; here all of them
@@ -97,13 +97,14 @@ __device__ __forceinline__ double invit_start(uint64_t j, uint64_t i) {
 }
 
 __global__ void __launch_bounds__(32)
-    k_trid_invit(int n, int m, int j0, const double *__restrict__ d, const double *__restrict__ e,
+    k_trid_invit(int n, int m, const int *__restrict__ num, const double *__restrict__ d, const double *__restrict__ e,
                  const double *__restrict__ shift, double tiny, InvitWork W, double *__restrict__ Z, long long ldz) {
   constexpr int U = 8;
   const int c = blockIdx.x * 32 + threadIdx.x;
   if (c >= m) return;
   const size_t M = (size_t)m;
-  const double lam = shift[j0 + c];
+  const int j = num[c];
+  const double lam = shift[c];
   double *const u0 = W.u0 + c, *const u1 = W.u1 + c, *const u2 = W.u2 + c, *const ml = W.ml + c, *const x = W.x + c;
   unsigned char *const swp = W.swp + c;
   auto floor_tiny = [&](double v) { return fabs(v) < tiny ? (v < 0.0 ? -tiny : tiny) : v; };
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(32)
     }
     u0[(size_t)(n - 1) * M] = floor_tiny(dg);
   }
-  for (int i = 0; i < n; ++i) x[(size_t)i * M] = invit_start((uint64_t)(j0 + c), (uint64_t)i);
+  for (int i = 0; i < n; ++i) x[(size_t)i * M] = invit_start((uint64_t)j, (uint64_t)i);
   for (int it = 0; it < kInvitIters; ++it) {
     // forward: P L (xi: row i's value so far)
     double xi = x[0];
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(32)
       amax = amax > v ? amax : v;
     }
     if (amax == 0.0) {
-      x[(size_t)((j0 + c) % n) * M] = 1.0;
+      x[(size_t)(j % n) * M] = 1.0;
       amax = 1.0;
     }
     double nrm = 0.0;
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(32)
     if (fabs(v) > fabs(big)) big = v;
   }
   const double sgn = big < 0.0 ? -1.0 : 1.0;
-  double *z = Z + (long long)(j0 + c) * ldz;
+  double *z = Z + (long long)j * ldz;
 #pragma unroll 8
   for (int i = 0; i < n; ++i) z[i] = __dmul_rn(sgn, x[(size_t)i * M]);
 }
@@ -401,24 +402,28 @@ int evslcu_trid_eigvals_async_wait(double *w) {
   return 0;
 }
 
-int evslcu_trid_invit(int n, const double *d, const double *e, int m, const double *shift, double tiny, double *Z,
-                      long long ldz) {
-  if (n < 2 || m < 1 || !d || !e || !shift || !Z) return fail(EVSLCU_ERR_ARG, "trid_invit: bad arguments");
-  const size_t row = 5 * sizeof(double) + 1;
-  const int chunk = (int)std::max<size_t>(32, std::min<size_t>((size_t)m, kInvitBytes / (row * (size_t)n)));
-  const int mc = std::min(m, chunk);
-  const size_t in = (size_t)2 * n + m;
-  double *buf = (double *)evslcu_malloc(sizeof(double) * in + row * (size_t)n * mc);
-  if (!buf) return EVSLCU_ERR_NOMEM;
+int evslcu_trid_invit(int n, const double *d, const double *e, int m, const int *num, const double *shift, double tiny,
+                      double *Z, long long ldz) {
+  if (n < 2 || m < 1 || !d || !e || !num || !shift || !Z) return fail(EVSLCU_ERR_ARG, "trid_invit: bad arguments");
+  const size_t row = 5 * sizeof(double) + 1, in = (size_t)2 * n + 2 * (size_t)m;
+  // vectors of a launch: what kInvitBytes hold, fewer when memory is short
+  int mc = (int)std::min<size_t>((size_t)m, std::max<size_t>(32, kInvitBytes / (row * (size_t)n)));
+  double *buf = nullptr;
+  while (!(buf = (double *)evslcu_malloc(sizeof(double) * in + row * (size_t)n * mc))) {
+    if (mc <= 32) return EVSLCU_ERR_NOMEM;
+    mc = std::max(32, mc / 2);
+  }
   double *dd = buf, *de = buf + n, *ds = buf + 2 * (size_t)n, *w = buf + in;
+  int *dn = (int *)(ds + m);
   int rc = evslcu_h2d_async(dd, d, sizeof(double) * (size_t)n);
   if (!rc) rc = evslcu_h2d_async(de, e, sizeof(double) * (size_t)(n - 1));
   if (!rc) rc = evslcu_h2d_async(ds, shift, sizeof(double) * (size_t)m);
+  if (!rc) rc = evslcu_h2d_async(dn, num, sizeof(int) * (size_t)m);
   const size_t blk = (size_t)n * mc;
   const InvitWork W{w, w + blk, w + 2 * blk, w + 3 * blk, w + 4 * blk, (unsigned char *)(w + 5 * blk)};
   for (int j0 = 0; j0 < m && !rc; j0 += mc) {
     const int c = std::min(mc, m - j0);
-    k_trid_invit<<<(c + 31) / 32, 32, 0, stream()>>>(n, c, j0, dd, de, ds, tiny, W, Z, ldz);
+    k_trid_invit<<<(c + 31) / 32, 32, 0, stream()>>>(n, c, dn + j0, dd, de, ds + j0, tiny, W, Z, ldz);
     count_launch();
     rc = check_launch("k_trid_invit");
   }

@@ -53,6 +53,9 @@ uint64_t evslcu_launch_count(void);
 /* ---- memory ------------------------------------------------------------- */
 void *evslcu_malloc(size_t nbytes);
 int evslcu_free(void *p);
+/* Requests above nbytes fail as on a full device (tests of what callers do
+ * then); 0: no limit. */
+int evslcu_set_malloc_limit(size_t nbytes);
 int evslcu_h2d(void *dst, const void *src, size_t nbytes);  /* synchronous */
 int evslcu_d2h(void *dst, const void *src, size_t nbytes);  /* synchronous */
 int evslcu_d2d(void *dst, const void *src, size_t nbytes);  /* async */
@@ -387,12 +390,13 @@ int evslcu_trid_eigvals_above(int k, const double *d, const double *e, double xm
 int evslcu_trid_eigvals_async(int k, const double *d, const double *e, double xmin);
 int evslcu_trid_eigvals_async_ready(void);
 int evslcu_trid_eigvals_async_wait(double *w);
-/* Eigenvectors by inverse iteration at the m shifts (ascending, on the host, as
- * d and e) of the symmetric tridiagonal matrix, into the columns of Z (device,
- * leading dimension ldz): the host's arithmetic, one thread per vector, no
- * orthogonalisation among them. */
-int evslcu_trid_invit(int n, const double *d, const double *e, int m, const double *shift, double tiny, double *Z,
-                      long long ldz);
+/* Eigenvectors number num[0..m-1] of the symmetric tridiagonal matrix by inverse
+ * iteration at their shifts (host arrays, as d and e), into the columns num[]
+ * of Z (device, leading dimension ldz): the host's arithmetic, one thread per
+ * vector, no orthogonalisation among them.  EVSLCU_ERR_NOMEM when there is no
+ * scratch for 32 vectors. */
+int evslcu_trid_invit(int n, const double *d, const double *e, int m, const int *num, const double *shift, double tiny,
+                      double *Z, long long ldz);
 /* Pattern tables read from the constant-memory pool when they fit there (1,
  * default) or always from global memory (0).  Same arithmetic either way. */
 int evslcu_set_pattern_const(int on);

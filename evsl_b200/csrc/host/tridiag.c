@@ -208,8 +208,8 @@ typedef struct {
   int n, ldz, j0, j1, rc;
   const double *d, *e, *shift;
   const int *cst;
+  const int *col; /* column of Z of each vector, -1: not computed here (null: its number) */
   double *Z, tiny;
-  int zfirst; /* the vector in Z's first column */
 } invit_job;
 
 static int invit_range(invit_job *jb) {
@@ -227,6 +227,8 @@ static int invit_range(invit_job *jb) {
   double *dg = buf, *du = buf + n, *u0 = buf + 2 * n, *u1 = buf + 3 * n, *u2 = buf + 4 * n, *ml = buf + 5 * n,
          *x = buf + 6 * n;
   for (int j = jb->j0; j < jb->j1; j++) {
+    const int zj_col = jb->col ? jb->col[j] : j;
+    if (zj_col < 0) continue;
     const double lam = jb->shift[j];
     const int cstart = jb->cst[j];
     /* LU with partial pivoting of T - lam I */
@@ -279,7 +281,7 @@ static int invit_range(invit_job *jb) {
       /* orthogonalise against the earlier vectors of the cluster (twice) */
       for (int pass = 0; pass < 2 && cstart < j; pass++) {
         for (int q = cstart; q < j; q++) {
-          const double *zq = Z + (size_t)(q - jb->zfirst) * ldz;
+          const double *zq = Z + (size_t)(jb->col ? jb->col[q] : q) * ldz;
           double dot = 0.0;
           for (int i = 0; i < n; i++) dot += zq[i] * x[i];
           for (int i = 0; i < n; i++) x[i] -= dot * zq[i];
@@ -303,7 +305,7 @@ static int invit_range(invit_job *jb) {
     for (int i = 1; i < n; i++)
       if (fabs(x[i]) > fabs(x[imax])) imax = i;
     const double sgn = (x[imax] < 0.0) ? -1.0 : 1.0;
-    double *zj = Z + (size_t)(j - jb->zfirst) * ldz;
+    double *zj = Z + (size_t)zj_col * ldz;
     for (int i = 0; i < n; i++) zj[i] = sgn * x[i];
   }
   free(buf);
@@ -348,52 +350,44 @@ static double invit_shifts(int n, const double *d, const double *e, int m, const
   return tnorm;
 }
 
-/* evsl_trid_eigvecs with the vectors on the device (Z: n x m, ld n): on the GPU,
- * bit for bit the host's, except clusters of close eigenvalues, whose vectors
- * are orthogonalised one after another -- those on the host, then copied. */
-int evsl_trid_eigvecs_device(int n, const double *d, const double *e, int m, const double *w, double *Z) {
-  if (m <= 0 || n <= 0) return 0;
-  if (n < 2) {
-    double *one = (double *)malloc(sizeof(double) * (size_t)m);
-    if (!one) return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-    for (int j = 0; j < m; j++) one[j] = 1.0;
-    const int rc1 = evslcu_h2d(Z, one, sizeof(double) * (size_t)m);
-    free(one);
-    return rc1 ? evsl_seterr(rc1, "%s", evslcu_errstr()) : 0;
+/* The vectors with col[j] >= 0 (all of them when col is null), in ranges split
+ * at cluster starts over host threads; every vector is computed the same way
+ * whatever the split. */
+static int invit_threads(int n, int ldz, int m, const double *d, const double *e, const double *shift, const int *cst,
+                         const int *col, double *Z, double tiny) {
+  int total = m;
+  if (col) {
+    total = 0;
+    for (int j = 0; j < m; j++) total += col[j] >= 0;
   }
-  double *shift = (double *)malloc(sizeof(double) * (size_t)m);
-  int *cst = (int *)malloc(sizeof(int) * (size_t)m);
-  if (!shift || !cst) {
-    free(shift);
-    free(cst);
-    return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-  }
-  const double tnorm = invit_shifts(n, d, e, m, w, shift, cst);
-  int rc = evslcu_trid_invit(n, d, e, m, shift, DBL_EPSILON * tnorm, Z, n);
-  if (rc) rc = evsl_seterr(rc, "%s", evslcu_errstr());
-  for (int j0 = 0; j0 < m && !rc;) {
-    int j1 = j0 + 1;
-    while (j1 < m && cst[j1] == j0) j1++;
-    if (j1 - j0 > 1) {
-      /* Zc: the cluster's columns, addressed by their numbers in all m */
-      const size_t cnt = (size_t)(j1 - j0) * n;
-      double *Zc = (double *)malloc(sizeof(double) * cnt);
-      if (!Zc) {
-        rc = evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-      } else {
-        invit_job jb = {n, n, j0, j1, 0, d, e, shift, cst, Zc, DBL_EPSILON * tnorm, j0};
-        if (invit_range(&jb))
-          rc = evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-        else if ((rc = evslcu_h2d(Z + (size_t)j0 * n, Zc, sizeof(double) * cnt)))
-          rc = evsl_seterr(rc, "%s", evslcu_errstr());
-        free(Zc);
-      }
+  long nth = sysconf(_SC_NPROCESSORS_ONLN);
+  nth = evsl_min(evsl_min(nth, (long)INVIT_MAX_THREADS), ((long)total * n) / INVIT_MIN_WORK);
+  if (nth < 1) nth = 1;
+  invit_job jobs[INVIT_MAX_THREADS];
+  pthread_t tid[INVIT_MAX_THREADS];
+  int nj = 0, j0 = 0, done = 0;
+  for (int t = 0; t < nth && j0 < m; t++) {
+    const int upto = (t == nth - 1) ? total : (int)(((long)total * (t + 1)) / nth);
+    int j1 = j0;
+    while (j1 < m && (done < upto || cst[j1] != j1)) {
+      done += !col || col[j1] >= 0;
+      j1++;
     }
+    if (j1 == j0) continue;
+    jobs[nj++] = (invit_job){n, ldz, j0, j1, 0, d, e, shift, cst, col, Z, tiny};
     j0 = j1;
   }
-  free(shift);
-  free(cst);
-  return rc;
+  int started = 0;
+  for (int t = 1; t < nj; t++) {
+    if (pthread_create(&tid[t], NULL, invit_thread, &jobs[t]) != 0) break;
+    started = t;
+  }
+  if (nj > 0) jobs[0].rc = invit_range(&jobs[0]);
+  for (int t = 1; t <= started; t++) pthread_join(tid[t], NULL);
+  for (int t = started + 1; t < nj; t++) jobs[t].rc = invit_range(&jobs[t]); /* threads that did not start */
+  for (int t = 0; t < nj; t++)
+    if (jobs[t].rc) return jobs[t].rc;
+  return 0;
 }
 
 int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const double *w, double *Z, int ldz) {
@@ -404,42 +398,95 @@ int evsl_trid_eigvecs(int n, const double *d, const double *e, int m, const doub
   }
   double *shift = (double *)malloc(sizeof(double) * (size_t)m);
   int *cst = (int *)malloc(sizeof(int) * (size_t)m);
+  int rc = EVSLX_ERR_NOMEM;
+  if (shift && cst) {
+    const double tnorm = invit_shifts(n, d, e, m, w, shift, cst);
+    rc = invit_threads(n, ldz, m, d, e, shift, cst, NULL, Z, DBL_EPSILON * tnorm);
+  }
+  free(shift);
+  free(cst);
+  return rc ? evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory") : 0;
+}
+
+/* evsl_trid_eigvecs with the vectors on the device (Z: n x m, ld n), the same
+ * bits.  Vectors of clusters of close eigenvalues are orthogonalised one after
+ * another, on the host's threads; the others go to the GPU beside them, a
+ * thread per vector, when there are at least INVIT_GPU_MIN of them and the
+ * scratch for it can be had.  A vector is one chain of dependent operations:
+ * 1.2 us (few vectors) to 2.3 us (many) per row there, 0.055 on a host core, so
+ * that fewer are done sooner by one core: rows x vectors, host / GPU in us:
+ * 400 x 16 368 / 586, 400 x 64 1,329 / 646, 850 x 32 1,400 / 1,417, 850 x 500
+ * 22,140 / 2,167, 2,000 x 32 3,258 / 4,486, 2,000 x 64 6,521 / 4,483,
+ * 8,800 x 32 14,277 / 20,088, 8,800 x 64 28,766 / 20,062. */
+#define INVIT_GPU_MIN 48
+
+int evsl_trid_eigvecs_device(int n, const double *d, const double *e, int m, const double *w, double *Z) {
+  if (m <= 0 || n <= 0) return 0;
+  double *shift = (double *)malloc(sizeof(double) * 2 * (size_t)m);
+  int *cst = (int *)malloc(sizeof(int) * 3 * (size_t)m);
+  double *Zh = NULL;
+  int rc = 0;
   if (!shift || !cst) {
     free(shift);
     free(cst);
     return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
   }
-  const double tnorm = invit_shifts(n, d, e, m, w, shift, cst);
-  /* ranges split at cluster starts over host threads; every vector is
-   * computed the same way whatever the split */
-  long nth = sysconf(_SC_NPROCESSORS_ONLN);
-  nth = evsl_min(evsl_min(nth, (long)INVIT_MAX_THREADS), ((long)m * n) / INVIT_MIN_WORK);
-  invit_job jobs[INVIT_MAX_THREADS];
-  pthread_t tid[INVIT_MAX_THREADS];
-  int nj = 0, j0 = 0;
-  for (int t = 0; t < (nth > 1 ? nth : 1) && j0 < m; t++) {
-    int j1 = (t == nth - 1 || nth <= 1) ? m : (int)(((long)m * (t + 1)) / nth);
-    if (j1 < j0 + 1) j1 = j0 + 1;
-    while (j1 < m && cst[j1] != j1) j1++;
-    jobs[nj] = (invit_job){n, ldz, j0, j1, 0, d, e, shift, cst, Z, DBL_EPSILON * tnorm, 0};
-    nj++;
-    j0 = j1;
+  double *lone_shift = shift + m;
+  int *lone = cst + m, *col = cst + 2 * (size_t)m, nlone = 0, nhost = 0;
+  double tnorm = 1.0;
+  if (n > 1) {
+    tnorm = invit_shifts(n, d, e, m, w, shift, cst);
+    for (int j = 0; j < m; j++)
+      if (cst[j] == j && (j + 1 == m || cst[j + 1] == j + 1)) {
+        lone_shift[nlone] = shift[j];
+        lone[nlone++] = j;
+      }
+    if (nlone < INVIT_GPU_MIN) nlone = 0;
+    if (nlone > 0) rc = evslcu_trid_invit(n, d, e, nlone, lone, lone_shift, DBL_EPSILON * tnorm, Z, n);
+    if (rc == EVSLCU_ERR_NOMEM) {
+      nlone = 0;
+      rc = 0;
+    }
+    if (rc) {
+      rc = evsl_seterr(rc, "%s", evslcu_errstr());
+      free(shift);
+      free(cst);
+      return rc;
+    }
   }
-  int started = 0;
-  for (int t = 1; t < nj; t++) {
-    if (pthread_create(&tid[t], NULL, invit_thread, &jobs[t]) != 0) break;
-    started = t;
+  for (int j = 0, l = 0; j < m; j++) {
+    if (l < nlone && lone[l] == j) {
+      col[j] = -1;
+      l++;
+    } else {
+      col[j] = nhost++;
+    }
   }
-  jobs[0].rc = invit_range(&jobs[0]);
-  for (int t = 1; t <= started; t++) pthread_join(tid[t], NULL);
-  for (int t = started + 1; t < nj; t++) jobs[t].rc = invit_range(&jobs[t]); /* threads that did not start */
-  int rc = 0;
-  for (int t = 0; t < nj; t++)
-    if (jobs[t].rc) rc = jobs[t].rc;
+  if (nhost > 0) {
+    Zh = (double *)malloc(sizeof(double) * (size_t)n * nhost);
+    if (!Zh) {
+      rc = EVSLX_ERR_NOMEM;
+    } else if (n == 1) {
+      for (int j = 0; j < m; j++) Zh[j] = 1.0;
+    } else {
+      rc = invit_threads(n, n, m, d, e, shift, cst, col, Zh, DBL_EPSILON * tnorm);
+    }
+    if (rc) rc = evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
+  }
+  /* a copy for each run of host vectors (pageable memory: read when the call returns) */
+  for (int j = 0; j < m && !rc;) {
+    int j1 = j + 1;
+    if (col[j] >= 0) {
+      while (j1 < m && col[j1] >= 0) j1++;
+      rc = evslcu_h2d_async(Z + (size_t)j * n, Zh + (size_t)col[j] * n, sizeof(double) * (size_t)n * (j1 - j));
+      if (rc) rc = evsl_seterr(rc, "%s", evslcu_errstr());
+    }
+    j = j1;
+  }
+  free(Zh);
   free(shift);
   free(cst);
-  if (rc) return evsl_seterr(EVSLX_ERR_NOMEM, "inverse iteration: out of memory");
-  return 0;
+  return rc;
 }
 
 /* Dense symmetric eigensolver.  A (n x n, column-major, lda) is read from

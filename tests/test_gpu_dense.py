@@ -8,6 +8,8 @@ numpy (1e-13 of the largest |C| entry): aligned and unaligned operands (odd
 leading dimensions), ragged edges, beta 0 and 0.5.
 """
 import ctypes as C
+import os
+import time
 
 import numpy as np
 import pytest
@@ -153,3 +155,57 @@ def test_tridiagonal_eigenvectors_on_gpu_are_the_hosts(gpu_lib, n, m, kind):
     assert lib.evsl_trid_eigvecs(n, vp(d), vp(e), m, vp(sel), vp(Z), n) == 0
     assert lib.evsl_trid_eigvecs_device(n, vp(d), vp(e), m, vp(sel), C.c_void_p(dZ.ptr)) == 0
     assert np.array_equal(dZ.to_host(shape=Z.shape), Z)
+
+
+def _eigvec_functions(lib):
+    for f in (lib.evsl_trid_eigvecs, lib.evsl_trid_eigvecs_device, lib.evsl_trid_eigvals):
+        f.restype = C.c_int
+    lib.evsl_trid_eigvals.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.evsl_trid_eigvecs.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int]
+    lib.evsl_trid_eigvecs_device.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+    lib.evslcu_set_malloc_limit.argtypes = [C.c_size_t]
+    return lambda a: a.ctypes.data_as(C.c_void_p)
+
+
+@pytest.mark.parametrize("limit", [0, 2 << 20, 1 << 16])
+def test_tridiagonal_eigenvectors_without_device_scratch(gpu_lib, limit):
+    """With room for only some of the vectors at a time, and with room for none
+    (the host's routine then), the vectors are the same; 30 pairs of close
+    eigenvalues lie among lone ones."""
+    lib = gpu_lib.lib
+    vp = _eigvec_functions(lib)
+    n, m = 600, 300
+    rng = np.random.default_rng(7)
+    d, e = rng.uniform(-0.1, 1.0, n), rng.uniform(0.01, 0.3, n)
+    w = np.zeros(n)
+    assert lib.evsl_trid_eigvals(n, vp(d), vp(e), vp(w)) == 0
+    sel = np.ascontiguousarray(w[n - m:])
+    sel[5:300:10] = sel[4:299:10] + 1e-9
+    Z = np.zeros((m, n))
+    assert lib.evsl_trid_eigvecs(n, vp(d), vp(e), m, vp(sel), vp(Z), n) == 0
+    dZ = evsl_b200.DeviceBuffer(lib, Z.nbytes)
+    try:
+        lib.evslcu_set_malloc_limit(limit)
+        assert lib.evsl_trid_eigvecs_device(n, vp(d), vp(e), m, vp(sel), C.c_void_p(dZ.ptr)) == 0
+    finally:
+        lib.evslcu_set_malloc_limit(0)
+    assert np.array_equal(dZ.to_host(shape=Z.shape), Z)
+
+
+@pytest.mark.skipif((os.cpu_count() or 1) < 4, reason="needs host cores to share the work")
+def test_clustered_eigenvectors_share_the_host_threads(gpu_lib):
+    """Vectors of clusters (here all: every eigenvalue is fourfold) are computed
+    by several host threads: more processor time than time."""
+    lib = gpu_lib.lib
+    vp = _eigvec_functions(lib)
+    n = 3000  # n vectors of n rows: work for four threads
+    rng = np.random.default_rng(8)
+    b = n // 4
+    d, e = np.tile(rng.uniform(-0.1, 1.0, b), 4), np.tile(np.r_[rng.uniform(0.01, 0.3, b - 1), 0.0], 4)
+    w = np.zeros(n)
+    assert lib.evsl_trid_eigvals(n, vp(d), vp(e), vp(w)) == 0
+    dZ = evsl_b200.DeviceBuffer(lib, 8 * n * n)
+    t, c = time.perf_counter(), time.process_time()
+    assert lib.evsl_trid_eigvecs_device(n, vp(d), vp(e), n, vp(w), C.c_void_p(dZ.ptr)) == 0
+    t, c = time.perf_counter() - t, time.process_time() - c
+    assert c > 1.5 * t, (c, t)
