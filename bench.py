@@ -116,7 +116,8 @@ def parse():
     p.add_argument("--filter-kernel", default="auto",
                    help="single-vector FP64 filter kernel: auto (timed choice per matrix) or one of "
                         "sell-loop, sell-unrolled, pattern-global-unrolled, pattern-global-loop, "
-                        "pattern-constant-loop, pattern-constant-unrolled, pattern-constant-rowdesc (profiling runs)")
+                        "pattern-constant-loop, pattern-constant-unrolled, pattern-constant-rowdesc, panel, "
+                        "merged-stencil (profiling runs)")
     return p.parse_args()
 
 
@@ -343,11 +344,7 @@ def run_ours(args):
 
     # the slice matrix's storage and filter kernel, read before config 1 replaces the matrix
     storage = storage_desc(lib)
-    v_chosen, _ = lib.filter_kernel()
-    kname = lib.FILTER_KERNELS[v_chosen] if v_chosen >= 0 else "sell-loop"
-    if args.filter_kernel == "auto" and args.filter_mode == "per-degree" and lib.row_pattern_count() > 0:
-        kname = "merged-stencil"  # grid operators run on their merged stencil; the variants are timed beside it
-        storage["filter_kernel"] = kname
+    kname = (storage["filter_kernel"] if args.filter_mode == "per-degree" else None) or "sell-loop"
     config1 = run_config1_ours(lib, lstream) if world == 1 else None
 
     # aggregate over ranks
@@ -633,6 +630,8 @@ def storage_desc(lib):
     if npat:
         desc += "; row-pattern dictionary: %d patterns, 2-byte pattern id per row" % npat
     v, us = lib.filter_kernel()
+    if lib.filter_stencil():
+        v = lib.FILTER_KERNELS.index("merged-stencil")  # the others are timed for comparison
     return {"matrix": desc, "filter_kernel": lib.FILTER_KERNELS[v] if v >= 0 else None,
             "filter_grid_blocks": lib.filter_kernel_grid() or "one row per thread",
             "us_per_degree_step_by_kernel": {k: round(t, 3) for k, t in us.items()}}

@@ -312,6 +312,7 @@ def load():
         "evslx_set_filter_kernel": ([C.c_int], C.c_int),
         "evslx_filter_kernel": ([C.POINTER(C.c_double)], C.c_int),
         "evslx_filter_kernel_grid": ([], C.c_int),
+        "evslx_filter_stencil": ([], C.c_int),
         "evslx_set_filter_wave": ([C.c_int], C.c_int),
         "evslx_get_filter_variant": ([], C.c_int),
         "evslx_tuned_filter_variant": ([C.c_int, C.c_int], C.c_int),
@@ -596,7 +597,8 @@ class Library:
         return int(self.lib.evslx_row_pattern_count())
 
     FILTER_KERNELS = ("sell-loop", "sell-unrolled", "pattern-global-unrolled", "pattern-global-loop",
-                      "pattern-constant-loop", "pattern-constant-unrolled", "pattern-constant-rowdesc", "panel")
+                      "pattern-constant-loop", "pattern-constant-unrolled", "pattern-constant-rowdesc", "panel",
+                      "merged-stencil")
 
     def set_filter_kernel(self, variant):
         """Force a single-vector filter kernel (index or name), or -1/None for timed selection."""
@@ -607,10 +609,15 @@ class Library:
         self._check(self.lib.evslx_set_filter_kernel(int(variant)), "evslx_set_filter_kernel")
 
     def filter_kernel(self):
-        """(chosen variant or -1, {variant name: measured us per degree step}) of the registered matrix."""
+        """(variant chosen by timing or -1, {variant name: measured us per degree step}) of the registered matrix;
+        see filter_stencil()."""
         us = (C.c_double * 8)()
         v = int(self.lib.evslx_filter_kernel(us))
         return v, {self.FILTER_KERNELS[i]: us[i] for i in range(8) if us[i] > 0}
+
+    def filter_stencil(self):
+        """Whether filters of one vector run on the registered matrix's merged stencil."""
+        return bool(self.lib.evslx_filter_stencil())
 
     def filter_kernel_grid(self):
         """Blocks per degree step chosen with the filter kernel (0: one row per thread)."""

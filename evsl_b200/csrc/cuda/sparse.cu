@@ -1102,8 +1102,8 @@ int evslcu::chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, d
 //   0  SELL-32, loop form            1  SELL-32, unrolled
 //   2  pattern table (global), unrolled   3  pattern table (global), loop form
 //   4  pattern table (constant), loop form  5  pattern table (constant), unrolled
-//   6  the merged stencil (stencil.cu) or, for a dictionary that does not merge
-//      into one, the constant table through per-row descriptors
+//   6  constant table through per-row descriptors
+//   7  column panels (panel.cu)            8  the merged stencil (stencil.cu)
 // Which is fastest depends on the size of the matrix (latency-bound small
 // operators favour the unrolled forms, L2-bound large ones the constant
 // table), so the first filter call on a matrix times every allowed variant on
@@ -1112,7 +1112,7 @@ int evslcu::chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, d
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kChebVariants = 8;
+constexpr int kChebVariants = 9, kChebStencil = 8;
 int g_cheb_force = -1;
 
 bool cheb_variant_ok(const evslcu_mat *A, int v) {
@@ -1126,8 +1126,9 @@ bool cheb_variant_ok(const evslcu_mat *A, int v) {
     case 3: return pat;
     case 4: return pconst;
     case 5: return pconst && unroll_width(A->pat_maxlen) > 0;
-    case 6: return stencil_ok(A) || (pconst && A->pat_desc);
+    case 6: return pconst && A->pat_desc;
     case 7: return A->pn64 != nullptr;
+    case kChebStencil: return stencil_ok(A);
     default: return false;
   }
 }
@@ -1157,8 +1158,8 @@ int launch_variant(const evslcu_mat *A, int v, bool first, bool epi, const doubl
       return panel_cheb_step(A, first, e, vk, vkm1, out, y, t, ncc, s, mu0, e ? ep->zold : nullptr,
                              e ? ep->nbeta : 0.0, e ? ep->dotv : nullptr, e ? ep->dot_out : nullptr);
     }
+    case kChebStencil: return stencil_step(A, first, vk, vkm1, out, y, t, ncc, s, mu0, epi ? ep : nullptr);
     case 6:
-      if (stencil_ok(A)) return stencil_step(A, first, vk, vkm1, out, y, t, ncc, s, mu0, epi ? ep : nullptr);
       if (A->pat_f32)
         return launch_cheb_step(PatCDView<true>{n, A->pat_desc}, n, 0, first, epi, vk, vkm1, out, y, t, ncc, s, mu0,
                                 ep);
@@ -1193,7 +1194,7 @@ float time_variant(const evslcu_mat *A, int v, int g, double *scr, cudaEvent_t e
 // Times every allowed variant on zero-filled scratch vectors and keeps the
 // fastest in A->cheb_variant, then its best grid limit in A->cheb_grid.
 int tune_cheb(evslcu_mat *A) {
-  static const int pref[kChebVariants] = {4, 6, 2, 3, 1, 0, 5, 7};
+  static const int pref[] = {4, 6, 2, 3, 1, 0, 5, 7};
   int fallback = 0;
   for (int v : pref)
     if (cheb_variant_ok(A, v)) {
@@ -1214,7 +1215,7 @@ int tune_cheb(evslcu_mat *A) {
   int rc = evslcu_memset(scr, 0, sizeof(double) * 3 * (size_t)n);
   if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = EVSLCU_ERR_CUDA;
   for (int v = 0; v < kChebVariants && !rc; ++v) {
-    if (!cheb_variant_ok(A, v)) continue;
+    if (!cheb_variant_ok(A, v) || v == kChebStencil) continue;
     const float us = time_variant(A, v, 0, scr, e0, e1, &rc);
     if (us > 0.0f) {
       A->cheb_us[v] = us;
@@ -1272,7 +1273,7 @@ int evslcu::chebav_per_degree(const evslcu_mat *A, const double *mu, int deg, do
   const int n = A->n;
   const double t1 = 1.0 / dd, t2 = 2.0 / dd, ncc = -cc;
   double *W[2] = {work, work + n};
-  if (stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == 6)) {
+  if (stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == kChebStencil)) {
     const_cast<evslcu_mat *>(A)->cheb_ran = 1;
     return stencil_chebav(A, mu, deg, cc, dd, v, y, work, epi);
   }
@@ -1344,8 +1345,12 @@ int evslcu_mat_cheb_variant(const evslcu_mat *A, float *us) {
   // times are asked for
   if (A->cheb_variant < 0 && A->cheb_ran) cheb_variant(A);
   if (us)
-    for (int v = 0; v < kChebVariants; ++v) us[v] = A->cheb_us[v];
+    for (int v = 0; v < kChebStencil; ++v) us[v] = A->cheb_us[v];
   return A->cheb_variant;
+}
+
+int evslcu_mat_cheb_stencil(const evslcu_mat *A) {
+  return A && stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == kChebStencil) ? 1 : 0;
 }
 
 int evslcu_set_cheb_max_grid(int blocks) {

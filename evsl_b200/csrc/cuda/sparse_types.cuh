@@ -109,7 +109,7 @@ struct evslcu_mat {
   int cheb_ran = 0;           // 1: the single-vector filter has run on the merged stencil
   unsigned char mf_ran[2][5] = {};  // the same for the multi-column filter, per (fp32, log2 B)
   int cheb_variant = -1;      // single-vector filter kernel chosen by timing (-1: not yet)
-  float cheb_us[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // measured time per degree step of each variant
+  float cheb_us[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // measured time per degree step of each variant
   int cheb_grid = 0;                      // tuned block limit per degree step (0: one row per thread)
   float cheb_best_us = 0.0f;              // time per degree step of the chosen variant and grid
 };

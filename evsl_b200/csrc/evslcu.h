@@ -401,19 +401,21 @@ int evslcu_trid_invit(int n, const double *d, const double *e, int m, const int 
  * default) or always from global memory (0).  Same arithmetic either way. */
 int evslcu_set_pattern_const(int on);
 /* Single-vector filter kernel variant: -1 (default) times the allowed
- * variants on a matrix's first filter call and keeps the fastest; 0..6 forces
+ * variants on a matrix's first filter call and keeps the fastest; 0..8 forces
  * one (0/1 SELL-32 loop/unrolled, 2/3 pattern table in global memory
  * unrolled/loop, 4/5 pattern table in constant memory loop/unrolled, 6 the
- * merged stencil, or without one the constant table addressed by a per-row
- * descriptor).  All give identical
- * results. */
+ * constant table addressed by a per-row descriptor, 7 column panels, 8 the
+ * merged stencil, which is used untimed where there is one).  All give
+ * identical results. */
 int evslcu_set_cheb_variant(int v);
 /* At most this many blocks per degree step of the single-vector filter
  * (0, default: one row per thread); rows beyond go round a grid-stride loop. */
 int evslcu_set_cheb_max_grid(int blocks);
-/* A's chosen variant (-1: not chosen yet) and, in us[0..6], the measured
+/* A's chosen variant (-1: not chosen yet) and, in us[0..7], the measured
  * microseconds per degree step of each variant timed (0: not timed). */
 int evslcu_mat_cheb_variant(const evslcu_mat *A, float *us);
+/* 1: A's single-vector filter runs on its merged stencil. */
+int evslcu_mat_cheb_stencil(const evslcu_mat *A);
 /* Column-panel layout for large general matrices (panel.cu): on/off, the
  * fewest rows for which it is built (0 keeps the current minimum, 2^18) and
  * the widest panel tried (0 keeps the current width, 16384 columns). */

@@ -501,6 +501,8 @@ int evslx_filter_kernel(double *us) {
   return v;
 }
 
+int evslx_filter_stencil(void) { return evslh.mat ? evslcu_mat_cheb_stencil(evslh.mat) : 0; }
+
 int evslx_set_panel_filter(int on, int min_rows, int max_width) {
   return from_cu(evslcu_set_panels(on, min_rows, max_width));
 }

@@ -177,24 +177,28 @@ int evslx_set_row_patterns(int on);
 int evslx_row_pattern_count(void);
 /* Kernel of the FP64 single-vector filter.  variant -1 (default): the first
  * filter call on a matrix times each variant allowed for it and keeps the
- * fastest; 0..6 forces one: 0/1 SELL-32 with looped/unrolled row products,
+ * fastest; 0..8 forces one: 0/1 SELL-32 with looped/unrolled row products,
  * 2/3 pattern table in global memory unrolled/looped, 4/5 pattern table in
- * constant memory looped/unrolled, 6 the merged stencil (a bit mask per row
- * over one short list of entries) where the dictionary merges into one of at
- * most 32 entries, else the constant-memory table addressed by a 4-byte
- * descriptor per row, 7 the column-panel layout (2-6 need the
+ * constant memory looped/unrolled, 6 constant-memory table addressed by a
+ * 4-byte descriptor per row, 7 the column-panel layout, 8 the merged stencil:
+ * a bit mask per row over one list of at most 32 entries (2-6 and 8 need the
  * row-pattern dictionary, 4-6 its table in the constant pool, 7 the panel
- * layout; filtering fails with EVSLX_ERR_ARG when the forced variant is not
- * available).  With no variant forced, a matrix with a merged stencil runs on
- * it (small ones in one launch for all degrees) without timing the others;
- * asking for the times (evslx_filter_kernel) times them.  Every variant gives
- * the same result bit for bit. */
+ * layout, 8 a dictionary that merges into such a list; filtering fails with
+ * EVSLX_ERR_ARG when the forced variant is not available).  With no variant
+ * forced, a matrix with a merged stencil runs on it (small ones in one launch
+ * for all degrees) without timing the others.  Every variant gives the same
+ * result bit for bit. */
 int evslx_set_filter_kernel(int variant);
-/* The registered matrix's chosen variant (-1: not chosen yet) and, when us is
- * not NULL, us[0..7] = measured microseconds per degree step of each variant
- * timed (0: not timed).  Variant 7 is the column-panel kernel (see
- * evslx_set_panel_filter). */
+/* The variant that timing chose for the registered matrix (-1: not timed yet)
+ * and, when us is not NULL, us[0..7] = measured microseconds per degree step of
+ * each variant timed (0: not timed).  Variant 7 is the column-panel kernel (see
+ * evslx_set_panel_filter).  A matrix that has been filtered on its merged
+ * stencil (evslx_filter_stencil) has its other variants timed by this call, for
+ * information. */
 int evslx_filter_kernel(double *us);
+/* 1: filters of one vector on the registered matrix run on its merged stencil,
+ * whatever evslx_filter_kernel says; 0: on the variant forced or chosen. */
+int evslx_filter_stencil(void);
 /* Column-panel filter for large general sparse matrices (no counterpart in
  * the reference, whose SpMV is the CSR matvec SRC/spmat.c:257-298 or
  * cuSPARSE, :529-621).  On a matrix whose rows have unequal lengths (SELL-C-

@@ -312,3 +312,35 @@ def test_columns_in_place(gpu_lib, shift, shape, prec, blocks):
         assert np.array_equal(buf.to_host(shape=X.shape)[1 + shift:6 + shift], ref)
     finally:
         lib.evslcu_set_stencil_cluster(0)
+
+
+def test_forced_kernels_and_the_merged_stencil_are_told_apart(gpu_lib):
+    """On a small grid the merged stencil filters in one launch and every other
+    kernel in one per degree: forced, "merged-stencil" and the row-descriptor
+    kernel are the ones that run, filter_stencil() says which is used, and a
+    matrix without a merged stencil refuses it."""
+    grid = O.lap_csr(40, 39, 1)
+    wide = stencil_csr(2000, [(o, 1.0 / (50 + o)) for o in range(-20, 21)])
+    pol, mu = polynomial(gpu_lib, 9, 8.0)
+
+    def launches(kernel, v):
+        gpu_lib.set_filter_kernel(kernel)
+        gpu_lib.chebav(pol, v)  # (a first call may prepare the kernel's tables)
+        before = gpu_lib.launch_count()
+        gpu_lib.chebav(pol, v)
+        return gpu_lib.launch_count() - before
+
+    try:
+        gpu_lib.set_csr(*grid)
+        v = O.seeded_normal(1560, 3)
+        assert gpu_lib.filter_stencil()
+        assert launches(None, v) == 1 and launches("merged-stencil", v) == 1 and gpu_lib.filter_stencil()
+        for kernel in ("sell-loop", "pattern-constant-rowdesc", "pattern-global-loop"):
+            assert launches(kernel, v) == 9 and not gpu_lib.filter_stencil(), kernel
+        gpu_lib.set_filter_kernel(None)
+        gpu_lib.set_csr(*wide)
+        assert gpu_lib.row_pattern_count() > 0 and not gpu_lib.filter_stencil()
+        with pytest.raises(E.EvslError, match="not available"):
+            launches("merged-stencil", O.seeded_normal(2000, 3))
+    finally:
+        gpu_lib.set_filter_kernel(None)
