@@ -339,17 +339,22 @@ __global__ void k_st_float(int n, const double *__restrict__ x, float *out) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) out[r] = (float)x[r];
 }
 
-// Two rows per thread: several columns from kStTwoRows rows on; one column where
-// one row per thread would need more blocks than run at once (6 on an SM).
+// Two rows per thread: FP64 columns and probes from kStTwoRows rows on; FP32
+// columns also, and one column only, where one row per thread would need more
+// blocks than run at once (6 on an SM).
 // Measured, us a degree of one column, 1 / 2 rows per thread: 215 thousand rows
 // 2.73 / 3.41, 343 thousand 3.57 / 3.56, 450 thousand 3.81 / 4.17, 592 thousand
 // 4.50 / 4.59, 10^6 (3-D) 6.35 / 6.49, 10^6 (2-D) 5.74 / 5.37, 4.1 million
-// 25.3 / 25.3; three rows were 4-8% slower than two at every size.
+// 25.3 / 25.3; three rows were 4-8% slower than two at every size.  FP32 columns
+// of a 5-point operator: 100 thousand rows x 16 9.82 / 7.43 (the packing kernel
+// 8.64), x 4 3.76 / 3.14, 40 thousand x 8 3.55 / 3.16; FP64, 9 points: 100
+// thousand x 16 10.5 / 10.7, x 4 4.08 / 4.84.
 constexpr int kStTwoRows = 150000;
+bool st_over_one_wave(long long rows) { return rows > 6LL * kThreads * sm_count(); }
 
-StMarch st_march(int n, int span, bool sym, bool one_column) {
+StMarch st_march(int n, int span, bool sym, bool two) {
   StMarch M;
-  int J = (one_column ? n > 6 * kThreads * sm_count() : n >= kStTwoRows) ? 2 : 1;
+  int J = two ? 2 : 1;
   if (!sym || span < 1 || (long long)span * J > n || n > (1 << 29)) J = 1;
   M.S = J > 1 ? span : std::max(n, 1);
   M.J = J;
@@ -363,7 +368,7 @@ template <int D>
 int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y, double t,
             double ncc, const StY<double> &Y, bool last, const evslcu_cheb_epi *ep) {
   const StArg<double, D> S = st_arg<double, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], true);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], st_over_one_wave(A->n));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads);
   cfg.blockDim = dim3(kThreads);
@@ -1341,7 +1346,8 @@ bool cl_columns_pay(const evslcu_mat *A, size_t vb, int n, double *us = nullptr)
 template <class VT, int D>
 int st_cols_launch(const evslcu_mat *A, int na, const StStepCols<VT> &C, int k) {
   const StArg<VT, D> S = st_arg<VT, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], false);
+  const bool two = A->n >= kStTwoRows || (sizeof(VT) == 4 && st_over_one_wave((long long)A->n * na));
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], two);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads, na);
   cfg.blockDim = dim3(kThreads);
@@ -1481,7 +1487,7 @@ int kpm_cluster(const evslcu_mat *A, int steps, int nvec, const double *probes, 
 template <int D>
 int kpm_steps(const evslcu_mat *A, int steps, int nvec, const double *probes, double ctr, double wid, double *raw) {
   const StArg<double, D> S = st_arg<double, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], false);
+  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], A->n >= kStTwoRows);
   const size_t n = (size_t)A->n;
   const int grid = (M.cols + kThreads - 1) / kThreads;
   const int group = (int)std::max<size_t>(1, std::min<size_t>((size_t)nvec, kStColsBytes / (16 * n)));

@@ -63,6 +63,9 @@ SHAPES = {
     "two-rows-7": (160003, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
     "two-rows-dropped": (151000, [(-900, -1.0), (-30, 0.2), (-1, -1.0), (0, 6.0), (1, -1.0), (30, 0.2), (900, -1.0)], 7),
     "two-rows-9": (155555, box9(400), 0),
+    # five FP32 columns together are more than one wave of blocks
+    "two-rows-fp32-9": (57601, box9(240), 0),
+    "two-rows-fp32-dropped": (50001, [(-900, -1.0), (-30, 0.2), (-1, -1.0), (0, 6.0), (1, -1.0), (30, 0.2), (900, -1.0)], 7),
     # one column's threads take two rows from one wave of blocks on (227,328 rows)
     "one-wave-7": (227328, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
     "over-one-wave-7": (227329, [(-2900, -1.0), (-53, -1.0), (-1, -1.0), (0, 6.0), (1, -1.0), (53, -1.0), (2900, -1.0)], 0),
@@ -125,7 +128,8 @@ def test_dictionaries_that_do_not_merge_keep_the_other_kernels(gpu_lib):
         assert np.array_equal(gpu_lib.chebav(pol, v), O.cheb_av(pol.as_dict(), *m, v))
 
 
-MULTI = ["cluster-over", "dropped-7", "eleven", "box-9", "lopsided", "two-rows-5", "two-rows-dropped"]
+MULTI = ["cluster-over", "dropped-7", "eleven", "box-9", "lopsided", "two-rows-5", "two-rows-dropped",
+         "two-rows-fp32-9", "two-rows-fp32-dropped"]
 
 
 @pytest.mark.parametrize("blocks", [-1, 0])
