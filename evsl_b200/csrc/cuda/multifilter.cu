@@ -163,7 +163,7 @@ struct Split {
 // columns on the column-split copy (ranges of columns whose rows of the
 // block fit in L2), for large general matrices whose block does not.
 static int g_mf_variant = -1;
-constexpr int kMfVariants = 8;
+constexpr int kMfVariants = 8, kMfStencil = 8;
 
 // One degree of the recurrence for all columns: thread (row r, part q)
 // handles columns q*CPT .. q*CPT+CPT-1 of row r.  Rows run over the padded
@@ -850,7 +850,7 @@ int autotune(evslcu_mat *A, int fp32, int B) {
     cudaGetLastError();  // without the panel layout the SELL kernels serve
   if (B > 1 && xs_prepare(A, fp32, B)) cudaGetLastError();  // without the split copy the SELL kernels serve
   for (int v = 0; !rc && v < kMfVariants; ++v) {
-    if (g_mf_variant >= 0 && v != g_mf_variant) continue;  // a forced variant is only timed
+    if (g_mf_variant >= 0 && g_mf_variant != kMfStencil && v != g_mf_variant) continue;  // a forced variant is only timed
     if ((v == 4 || v == 5) && !mf_pattern_ok(A)) continue;
     if (v == 6 && !(B == 1 && (fp32 ? A->pn32 : A->pn64))) continue;
     if (v == 7 && !(B > 1 && xs_of(A, fp32, B))) continue;
@@ -901,9 +901,13 @@ int autotune(evslcu_mat *A, int fp32, int B) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   evslcu_free(buf);
+  // columns on a merged stencil that is not taken untimed
+  float st_us = 0.0f;
+  if (!rc && stencil_ok(A) && !stencil_plain(A)) rc = stencil_columns_time(A, fp32, B, &st_us);
   if (!rc) {
     slot = (signed char)bestv;
     A->mf_cost_us[fp32 ? 1 : 0][log2_width(B)] = 1000.0f * best / steps;
+    A->mf_st_us[fp32 ? 1 : 0][log2_width(B)] = st_us;
   }
   return rc;
 }
@@ -912,6 +916,20 @@ int autotune_groups(const evslcu_mat *A, int fp32, int ncols) {
   int rc = 0;
   for (int c0 = 0; !rc && c0 < ncols; c0 += kMaxB) rc = autotune((evslcu_mat *)A, fp32, group_width(std::min(kMaxB, ncols - c0)));
   return rc;
+}
+
+// Whether the columns run on the merged stencil (with the vectors' places
+// checked once they are known): forced, plain, or timed as faster.
+bool columns_on_stencil(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, bool vectors, int *rc) {
+  *rc = 0;
+  const bool ok = stencil_columns_ok(A, fp32, ncols, cols, vectors);
+  if (g_mf_variant == kMfStencil && !ok)
+    *rc = fail(EVSLCU_ERR_ARG, "filter variant %d is not available for this matrix or these columns", kMfStencil);
+  if (!ok || (g_mf_variant >= 0 && g_mf_variant != kMfStencil)) return false;
+  if (g_mf_variant == kMfStencil || stencil_plain(A)) return true;
+  if ((*rc = autotune_groups(A, fp32, ncols))) return false;
+  const int f = fp32 ? 1 : 0, b = log2_width(group_width(std::min(kMaxB, ncols)));
+  return A->mf_st_us[f][b] > 0.0f && A->mf_st_us[f][b] < A->mf_cost_us[f][b];
 }
 
 // The whole launch sequence for ncols columns; x and y pointers are read
@@ -1012,7 +1030,9 @@ int evslcu_filter_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu
   if (rc) return rc;
   if (!work || work_bytes < evslcu_filter_columns_work(A->n, fp32, ncols))
     return fail(EVSLCU_ERR_ARG, "filter_columns: work too small");
-  if (g_mf_variant < 0 && stencil_columns_ok(A, fp32, ncols, cols, true)) {
+  const bool on_stencil = columns_on_stencil(A, fp32, ncols, cols, true, &rc);
+  if (rc) return rc;
+  if (on_stencil) {
     std::vector<size_t> off((size_t)ncols);
     double *mu = stencil_columns_mu(ncols, cols, off.data(), &rc);
     if (!rc) rc = stencil_columns(A, fp32, ncols, cols, mu, off.data(), work);
@@ -1058,8 +1078,13 @@ evslcu_filter_plan *evslcu_filter_plan_create(const evslcu_mat *A, int fp32, int
     evslcu_filter_plan_destroy(P);
     return nullptr;
   }
-  if (g_mf_variant < 0 && stencil_columns_ok(A, fp32, ncols, cols, false)) {
-    int err = 0;
+  int err = 0;
+  const bool on_stencil = columns_on_stencil(A, fp32, ncols, cols, false, &err);
+  if (err) {
+    evslcu_filter_plan_destroy(P);
+    return nullptr;
+  }
+  if (on_stencil) {
     P->st_cols = (evslcu_filter_col *)malloc(sizeof(evslcu_filter_col) * (size_t)ncols);
     P->st_off = (size_t *)malloc(sizeof(size_t) * (size_t)ncols);
     if (P->st_cols && P->st_off) {
@@ -1072,7 +1097,7 @@ evslcu_filter_plan *evslcu_filter_plan_create(const evslcu_mat *A, int fp32, int
     }
     return P;
   }
-  int err = autotune_groups(A, fp32, ncols);
+  err = autotune_groups(A, fp32, ncols);
   P->coef = err ? nullptr : coef_build(fp32, ncols, cols, &err);
   if (!P->coef) {
     evslcu_filter_plan_destroy(P);
@@ -1129,7 +1154,7 @@ int evslcu_filter_plan_run(evslcu_filter_plan *P, const double *const *x, double
 int evslcu_filter_plan_columns(const evslcu_filter_plan *P) { return P ? P->ncols : 0; }
 
 int evslcu_set_filter_variant(int v) {
-  if (v < -1 || v >= kMfVariants) return fail(EVSLCU_ERR_ARG, "filter variant must be -1 (tuned) or 0..7");
+  if (v < -1 || v > kMfStencil) return fail(EVSLCU_ERR_ARG, "filter variant must be -1 (tuned) or 0..8");
   g_mf_variant = v;
   return 0;
 }
@@ -1145,7 +1170,7 @@ int evslcu_set_xs_range_bytes(long long bytes) {
 int evslcu_mat_filter_variant(const evslcu_mat *A, int fp32, int B) {
   if (!A) return -1;
   const int f = fp32 ? 1 : 0, b = log2_width(B);
-  // columns filtered on a merged stencil: the variants are timed when asked for
+  // columns filtered on a plain merged stencil: the variants are timed when asked for
   if (A->mf_variant[f][b] < 0 && A->mf_ran[f][b]) autotune(const_cast<evslcu_mat *>(A), fp32, group_width(std::min(B, kMaxB)));
   return A->mf_variant[f][b];
 }
@@ -1153,10 +1178,12 @@ int evslcu_mat_filter_variant(const evslcu_mat *A, int fp32, int B) {
 double evslcu_filter_step_cost(evslcu_mat *A, int fp32, int B) {
   if (!A || A->kernel != 0 || B < 1) return -1.0;
   if (fp32 && A->vfmt == 0 && !A->sval32) return -1.0;
-  if (g_mf_variant < 0 && stencil_ok(A)) return stencil_step_us(A, fp32, B);
+  if ((g_mf_variant < 0 && stencil_plain(A)) || (g_mf_variant == kMfStencil && stencil_ok(A)))
+    return stencil_step_us(A, fp32, B);
   const int Bp = group_width(std::min(B, kMaxB));
   if (autotune(A, fp32, Bp)) return -1.0;
-  return (double)A->mf_cost_us[fp32 ? 1 : 0][log2_width(Bp)];
+  const float us = A->mf_cost_us[fp32 ? 1 : 0][log2_width(Bp)], st = A->mf_st_us[fp32 ? 1 : 0][log2_width(Bp)];
+  return (double)(g_mf_variant < 0 && st > 0.0f ? std::min(us, st) : us);
 }
 
 void evslcu_filter_plan_destroy(evslcu_filter_plan *P) {

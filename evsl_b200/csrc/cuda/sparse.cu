@@ -1107,8 +1107,8 @@ int evslcu::chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, d
 // Which is fastest depends on the size of the matrix (latency-bound small
 // operators favour the unrolled forms, L2-bound large ones the constant
 // table), so the first filter call on a matrix times every allowed variant on
-// scratch vectors and keeps the fastest.  A matrix with a merged stencil needs
-// no timing: that form was the fastest at every size measured (stencil.cu).
+// scratch vectors and keeps the fastest.  A plain merged stencil needs no timing
+// (stencil_plain, stencil.cu).
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -1158,7 +1158,6 @@ int launch_variant(const evslcu_mat *A, int v, bool first, bool epi, const doubl
       return panel_cheb_step(A, first, e, vk, vkm1, out, y, t, ncc, s, mu0, e ? ep->zold : nullptr,
                              e ? ep->nbeta : 0.0, e ? ep->dotv : nullptr, e ? ep->dot_out : nullptr);
     }
-    case kChebStencil: return stencil_step(A, first, vk, vkm1, out, y, t, ncc, s, mu0, epi ? ep : nullptr);
     case 6:
       if (A->pat_f32)
         return launch_cheb_step(PatCDView<true>{n, A->pat_desc}, n, 0, first, epi, vk, vkm1, out, y, t, ncc, s, mu0,
@@ -1215,8 +1214,12 @@ int tune_cheb(evslcu_mat *A) {
   int rc = evslcu_memset(scr, 0, sizeof(double) * 3 * (size_t)n);
   if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = EVSLCU_ERR_CUDA;
   for (int v = 0; v < kChebVariants && !rc; ++v) {
-    if (!cheb_variant_ok(A, v) || v == kChebStencil) continue;
-    const float us = time_variant(A, v, 0, scr, e0, e1, &rc);
+    if (!cheb_variant_ok(A, v) || (v == kChebStencil && stencil_plain(A))) continue;
+    float us = 0.0f;
+    if (v == kChebStencil)
+      rc = stencil_time(A, &us);
+    else
+      us = time_variant(A, v, 0, scr, e0, e1, &rc);
     if (us > 0.0f) {
       A->cheb_us[v] = us;
       if (best_us == 0.0f || us < best_us) {
@@ -1229,7 +1232,7 @@ int tune_cheb(evslcu_mat *A) {
   // 16 / 8 blocks per SM going round a grid-stride loop
   A->cheb_grid = 0;
   for (int g : {16 * sm_count(), 8 * sm_count()}) {
-    if (rc || best_us == 0.0f) break;
+    if (rc || best_us == 0.0f || best == kChebStencil) break;
     const float us = time_variant(A, best, g, scr, e0, e1, &rc);
     if (us > 0.0f && us < best_us) {
       best_us = us;
@@ -1250,9 +1253,9 @@ int tune_cheb(evslcu_mat *A) {
 int cheb_variant(const evslcu_mat *A_) {
   evslcu_mat *A = const_cast<evslcu_mat *>(A_);
   if (A->kernel != 0) return -1;
-  // a matrix with a merged stencil claims constant memory only when the
+  // a matrix with a plain merged stencil claims constant memory only when the
   // variants that read it are asked for
-  if (A->st_d && A->pat_chdr < 0 && pat_const_claim(A)) return EVSLCU_ERR_CUDA;
+  if (A->st_plain && A->pat_chdr < 0 && pat_const_claim(A)) return EVSLCU_ERR_CUDA;
   if (g_cheb_force == 7 && panel_candidate(A) && !A->pn64) {
     const int prc = panel_build(A, 0);
     if (prc) return prc;
@@ -1273,11 +1276,10 @@ int evslcu::chebav_per_degree(const evslcu_mat *A, const double *mu, int deg, do
   const int n = A->n;
   const double t1 = 1.0 / dd, t2 = 2.0 / dd, ncc = -cc;
   double *W[2] = {work, work + n};
-  if (stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == kChebStencil)) {
-    const_cast<evslcu_mat *>(A)->cheb_ran = 1;
-    return stencil_chebav(A, mu, deg, cc, dd, v, y, work, epi);
-  }
-  const int var = cheb_variant(A);
+  const bool plain = g_cheb_force < 0 && stencil_plain(A);
+  if (plain) const_cast<evslcu_mat *>(A)->cheb_ran = 1;
+  const int var = plain ? kChebStencil : cheb_variant(A);
+  if (var == kChebStencil) return stencil_chebav(A, mu, deg, cc, dd, v, y, work, epi);
   if (var == -2) return fail(EVSLCU_ERR_ARG, "filter kernel variant %d is not available for this matrix", g_cheb_force);
   if (var <= EVSLCU_ERR_CUDA) return var;
   for (int k = 1; k <= deg; ++k) {
@@ -1333,7 +1335,7 @@ int evslcu_mat_cheb_grid(const evslcu_mat *A) { return A ? A->cheb_grid : 0; }
 
 double evslcu_chebav_step_cost(evslcu_mat *A) {
   if (!A || A->kernel != 0) return -1.0;
-  if (stencil_ok(A) && g_cheb_force < 0) return stencil_step_us(A, 0, 1);
+  if (stencil_plain(A) && g_cheb_force < 0) return stencil_step_us(A, 0, 1);
   const int v = cheb_variant(A);  // tunes on first use
   if (v < 0) return -1.0;
   return A->cheb_best_us > 0.0f ? (double)A->cheb_best_us : (double)A->cheb_us[v];
@@ -1341,8 +1343,8 @@ double evslcu_chebav_step_cost(evslcu_mat *A) {
 
 int evslcu_mat_cheb_variant(const evslcu_mat *A, float *us) {
   if (!A) return fail(EVSLCU_ERR_ARG, "null matrix");
-  // a matrix filtered on its merged stencil has its variants timed when the
-  // times are asked for
+  // a matrix filtered on its plain merged stencil has its variants timed when
+  // the times are asked for
   if (A->cheb_variant < 0 && A->cheb_ran) cheb_variant(A);
   if (us)
     for (int v = 0; v < kChebStencil; ++v) us[v] = A->cheb_us[v];
@@ -1350,7 +1352,9 @@ int evslcu_mat_cheb_variant(const evslcu_mat *A, float *us) {
 }
 
 int evslcu_mat_cheb_stencil(const evslcu_mat *A) {
-  return A && stencil_ok(A) && (g_cheb_force < 0 || g_cheb_force == kChebStencil) ? 1 : 0;
+  if (!A || !stencil_ok(A)) return 0;
+  return g_cheb_force == kChebStencil ||
+         (g_cheb_force < 0 && (stencil_plain(A) || A->cheb_variant == kChebStencil));
 }
 
 int evslcu_set_cheb_max_grid(int blocks) {
@@ -1431,7 +1435,7 @@ evslcu_mat *evslcu_mat_create(int n, int nnz, const int *ia, const int *ja, cons
     }
   }
   if (build_sell_device(M, g_compress != 0) || evslcu_sync() || (g_patterns && build_patterns_device(M)) ||
-      stencil_build(M) || (!M->st_d && pat_const_claim(M))) {
+      stencil_build(M) || (!M->st_plain && pat_const_claim(M))) {
     evslcu_mat_destroy(M);
     return nullptr;
   }
@@ -1479,7 +1483,7 @@ int evslcu_mat_get_kernel(const evslcu_mat *A) { return A ? A->kernel : -1; }
 int evslcu_spmv(const evslcu_mat *A, const double *x, double *y) {
   if (!A) return fail(EVSLCU_ERR_ARG, "null matrix");
   const int grid = grid_for(A->n);
-  if (stencil_ok(A)) return stencil_spmv(A, x, y, 1);
+  if (stencil_spmv_ok(A)) return stencil_spmv(A, x, y, 1);
   if (evslcu_mat_uses_patterns(A)) {
     if (A->pat_chdr >= 0 && g_pattern_const && A->pat_f32)
       k_spmv<PatCPView><<<grid, kThreads, 0, stream()>>>(PatCPView{A->n, A->pat_id, A->pat_chdr}, x, y);
@@ -1512,7 +1516,7 @@ int evslcu_spmv_cols(const evslcu_mat *A, const double *X, double *Y, int m) {
     const dim3 g(gx, mc);
     const double *Xc = X + (size_t)c0 * ld;
     double *Yc = Y + (size_t)c0 * ld;
-    if (stencil_ok(A)) {
+    if (stencil_spmv_ok(A)) {
       const int rc = stencil_spmv(A, Xc, Yc, mc);
       if (rc) return rc;
       continue;
@@ -1663,7 +1667,7 @@ static int kpm_dots_doubling(const evslcu_op *op, int n, int Mdeg, int nvec, con
                              double wid, double *dots) {
   const int B = nvec;
   const int K = (Mdeg + 1) / 2;
-  if (stencil_ok(op->A)) {
+  if (stencil_kpm_ok(op->A)) {
     const size_t count = (size_t)K * 3 * B;
     double *raw = (double *)evslcu_malloc(sizeof(double) * count);
     if (!raw) return fail(EVSLCU_ERR_NOMEM, "kpm: out of device memory");

@@ -65,6 +65,7 @@ struct evslcu_mat {
   void *sell_block = nullptr;  // one allocation holding scol and sval (L2 window)
   size_t sell_bytes = 0;
   void *sval32 = nullptr;  // FP32 copy of sval for the FP32 filter (when vfmt == 0)
+  float mf_st_us[2][5] = {};  // the merged stencil's columns beside mf_cost_us (0: not timed)
   signed char mf_variant[2][5] = {{-1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1}};  // tuned kernel per (fp32, log2 B)
   float mf_cost_us[2][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};  // its measured time per degree step
   long long bandwidth = 0;  // max |col - row| over the stored entries
@@ -97,6 +98,7 @@ struct evslcu_mat {
   int st_d = 0;
   int st_reach = 0;  // largest |offset|
   int st_span = 0;   // largest offset: rows r and r + st_span share most of what they gather
+  int st_plain = 0;  // 1: 5, 7 or 9 entries and a row that has them all
   void *st_mask = nullptr;
   double st_val[32] = {};
   int st_off[32] = {};
@@ -490,6 +492,11 @@ int chebav_user_matvec(const evslcu_op *op, const double *mu, int deg, double cc
 int stencil_build(evslcu_mat *M);
 void stencil_free(evslcu_mat *M);
 bool stencil_ok(const evslcu_mat *M);
+bool stencil_plain(const evslcu_mat *M);
+bool stencil_spmv_ok(const evslcu_mat *M);
+bool stencil_kpm_ok(const evslcu_mat *M);
+int stencil_time(const evslcu_mat *A, float *us);
+int stencil_columns_time(const evslcu_mat *A, int fp32, int ncols, float *us);
 bool stencil_columns_ok(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, bool vectors);
 double *stencil_columns_mu(int ncols, const evslcu_filter_col *cols, size_t *off, int *err);
 int stencil_columns(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, const double *dmu,
@@ -500,8 +507,6 @@ int stencil_batch(int ncols, const evslcu_batch_col *cols, unsigned char *done);
 int stencil_spmv(const evslcu_mat *A, const double *X, double *Y, int m);
 int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,
                    double *work, const evslcu_cheb_epi *epi);
-int stencil_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y,
-                 double t, double ncc, double s, double mu0, const evslcu_cheb_epi *epi);
 int launch_scale_copy(int n, double a, const double *x, double *y);
 int launch_lan_epi(int n, const evslcu_cheb_epi *epi, double *y);
 

@@ -1629,6 +1629,7 @@ int stencil_build(evslcu_mat *M) {
   M->st_mask = dm;
   M->st_reach = reach;
   M->st_span = span;
+  M->st_plain = (d == 5 || d == 7 || d == 9) && M->pat_maxlen == d;
   M->st_d = d;
   return 0;
 }
@@ -1636,7 +1637,7 @@ int stencil_build(evslcu_mat *M) {
 void stencil_free(evslcu_mat *M) {
   evslcu_free(M->st_mask);
   M->st_mask = nullptr;
-  M->st_d = 0;
+  M->st_d = M->st_plain = 0;
 }
 
 // Y(:, c) = A X(:, c) for m columns (1 <= m <= 65535).
@@ -1665,12 +1666,91 @@ void set_cluster_wait_limit(unsigned long long polls) {
 
 bool stencil_ok(const evslcu_mat *M) { return M->st_d > 0 && M->use_pat && M->kernel == 0; }
 
-// One degree step with y written at once (the kernel's timing among the other
-// variants).
-int stencil_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y,
-                 double t, double ncc, double s, double mu0, const evslcu_cheb_epi *epi) {
-  StY<double> Y{first ? 2 : 1, first ? 1 : 0, 0.0, mu0, s};
-  return st_step_any(A, first, vk, vkm1, out, y, t, ncc, Y, epi != nullptr, epi);
+// Whether filters take the merged stencil untimed: 5, 7 or 9
+// entries, all of them in some row.  These widths are compiled, and full rows
+// skip their masks; it was the fastest at every size measured (10^4 to 4.1
+// million rows, 1 to 16 columns, both precisions).  Where rows take only part
+// of a longer list, as with coefficients that vary, or the list is padded to
+// the next width, each row does the whole list's loads and multiplications, and
+// the stencil is one of the variants that a first filter times.  Us a degree on
+// 10^6 rows, fastest dictionary kernel / stencil: 5 points with 2 diagonal
+// values 6.80 / 6.76, with 5 6.92 / 8.16, with 6 sets of coefficients (30
+// entries) 6.89 / 23.9, 13 points 11.7 / 11.5, 27 points 21.6 / 25.6; on 10^4
+// rows 3.64 / 0.86, 2.66 / 0.94, 2.79 / 2.68, 3.61 / 2.68, 5.28 / 2.78.
+bool stencil_plain(const evslcu_mat *M) { return stencil_ok(M) && M->st_plain; }
+
+// Whether products take it: a list of 5 to 16 entries that some row has all of
+// (us for 16 columns, dictionary / stencil: 10^6 rows, 3 points 82.8 / 89.5, 5
+// points 93.6 / 94.7, 9 points 118 / 106, 13 points 165 / 154, 27 points 326 /
+// 590, 5 points with 6 sets of coefficients 93 / 540; 10^5 rows, 13 points 35.6
+// / 26.2).
+bool stencil_spmv_ok(const evslcu_mat *M) {
+  return stencil_ok(M) && M->st_d >= 5 && M->st_d <= 16 && M->st_d == M->pat_maxlen;
+}
+
+// Whether KPM runs on it: the dictionary's kernel reads the probes interleaved
+// and pays for each launch and reduction, so the list may be up to four times
+// as wide as a row (16 probes, us a step on 10^6 rows, dictionary / stencil: 30
+// entries in rows of 5 228 / 308, 28 in rows of 7 249 / 314, 10 in 5 228 / 167,
+// 26 in 13 539 / 322), and any width on small operators (10^5 rows, 30 in 5 32 /
+// 33, 10^4 14.3 / 7.3).
+bool stencil_kpm_ok(const evslcu_mat *M) {
+  return stencil_ok(M) && (M->n <= 65536 || st_width(M->st_d) <= 4 * M->pat_maxlen);
+}
+
+// Microseconds per degree of run(), a filter of degree kTimeDeg.
+constexpr int kTimeDeg = 24;
+template <class F>
+static int time_degrees(F &&run, float *us) {
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  float ms = 0.0f;
+  int rc = run();
+  if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
+    rc = fail(EVSLCU_ERR_CUDA, "stencil timing: no events");
+  if (!rc) cudaEventRecord(e0, stream());
+  if (!rc) rc = run();
+  if (!rc) cudaEventRecord(e1, stream());
+  if (!rc) rc = evslcu_sync();
+  if (!rc) cudaEventElapsedTime(&ms, e0, e1);
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  *us = 1e3f * ms / kTimeDeg;
+  return rc;
+}
+
+// The filter of one vector, timed on zero vectors; *us stays 0 without memory.
+int stencil_time(const evslcu_mat *A, float *us) {
+  const size_t n = (size_t)A->n;
+  *us = 0.0f;
+  double *w = (double *)evslcu_malloc(sizeof(double) * 4 * n);
+  if (!w) return 0;
+  const std::vector<double> mu((size_t)kTimeDeg + 1, 0.0);
+  int rc = evslcu_memset(w, 0, sizeof(double) * 4 * n);
+  if (!rc)
+    rc = time_degrees(
+        [&] { return stencil_chebav(A, mu.data(), kTimeDeg, 0.0, 1.0, w, w + n, w + 2 * n, nullptr); }, us);
+  evslcu_free(w);
+  return rc;
+}
+
+// The filter of ncols (at most kStCols) columns, likewise.
+int stencil_columns_time(const evslcu_mat *A, int fp32, int ncols, float *us) {
+  const size_t n = (size_t)A->n, work = evslcu_filter_columns_work(A->n, fp32, ncols);
+  *us = 0.0f;
+  double *w = (double *)evslcu_malloc(sizeof(double) * n * (ncols + 1) + work);
+  if (!w) return 0;
+  const std::vector<double> mu((size_t)kTimeDeg + 1, 0.0);
+  std::vector<evslcu_filter_col> cols((size_t)ncols);
+  std::vector<size_t> off((size_t)ncols);
+  for (int c = 0; c < ncols; ++c) cols[c] = evslcu_filter_col{mu.data(), kTimeDeg, 0.0, 1.0, w, w + n * (c + 1)};
+  int rc = evslcu_memset(w, 0, sizeof(double) * n);
+  double *dmu = rc ? nullptr : stencil_columns_mu(ncols, cols.data(), off.data(), &rc);
+  if (!rc)
+    rc = time_degrees(
+        [&] { return stencil_columns(A, fp32, ncols, cols.data(), dmu, off.data(), w + n * (ncols + 1)); }, us);
+  evslcu_free(dmu);
+  evslcu_free(w);
+  return rc;
 }
 
 int stencil_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double dd, const double *v, double *y,

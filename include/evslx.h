@@ -185,8 +185,9 @@ int evslx_row_pattern_count(void);
  * row-pattern dictionary, 4-6 its table in the constant pool, 7 the panel
  * layout, 8 a dictionary that merges into such a list; filtering fails with
  * EVSLX_ERR_ARG when the forced variant is not available).  With no variant
- * forced, a matrix with a merged stencil runs on it (small ones in one launch
- * for all degrees) without timing the others.  Every variant gives the same
+ * forced, a merged stencil of 5, 7 or 9 entries that some row has all of is used
+ * (on small matrices in one launch for all degrees) without timing the others;
+ * other merged stencils are timed with them.  Every variant gives the same
  * result bit for bit. */
 int evslx_set_filter_kernel(int variant);
 /* The variant that timing chose for the registered matrix (-1: not timed yet)
@@ -387,6 +388,12 @@ int evslx_chebav_multi(int ncols, const polparams *pols, const double *X, double
  * columns equal ChebAv bit for bit.  Needs increasing column indices in
  * every row; filtering fails with EVSLX_ERR_ARG when the matrix or width
  * has no such copy;
+ * 8 -- the merged stencil, columns apart: each column its own vectors, one
+ * launch per degree for up to 16 columns, or one for all degrees on small
+ * matrices.  Needs a merged stencil, degrees of at least 1 and results that do
+ * not overwrite other columns' vectors; filtering fails with EVSLX_ERR_ARG
+ * otherwise.  Used without timing where filters of one vector use it so
+ * (evslx_set_filter_kernel);
  * -1 (default) -- autotuned: the first filter on a matrix with a given
  * precision and block width times the variants available for it on a few
  * degree steps and keeps the fastest for that matrix. */

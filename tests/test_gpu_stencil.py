@@ -104,6 +104,7 @@ def test_stencil_filter_is_bitwise(gpu_lib, shape, blocks):
         pol, mu = polynomial(gpu_lib, deg, bound)
         try:
             gpu_lib.lib.evslcu_set_stencil_cluster(blocks)
+            gpu_lib.set_filter_kernel("merged-stencil")
             y = gpu_lib.chebav(pol, v)
             gpu_lib.set_filter_kernel(0)  # SELL storage, pinned to the oracle elsewhere
             assert np.array_equal(y, gpu_lib.chebav(pol, v)), deg
@@ -148,6 +149,7 @@ def test_stencil_columns_are_bitwise(gpu_lib, shape, prec, blocks):
     pols = [p for p, _ in made]
     try:
         gpu_lib.lib.evslcu_set_stencil_cluster(blocks)
+        gpu_lib.set_filter_variant(8)
         Y = gpu_lib.chebav_multi(pols, X, prec)
         gpu_lib.set_filter_variant(0)
         assert np.array_equal(Y, gpu_lib.chebav_multi(pols, X, prec))
@@ -348,3 +350,87 @@ def test_forced_kernels_and_the_merged_stencil_are_told_apart(gpu_lib):
             launches("merged-stencil", O.seeded_normal(2000, 3))
     finally:
         gpu_lib.set_filter_kernel(None)
+
+
+def _sets(n, offsets, sets):
+    """Rows of `offsets`, the values one of `sets` multiples by row range."""
+    ia, ja, a = stencil_csr(n, [(o, 5.0 if o == 0 else -1.0) for o in offsets])
+    rows = np.repeat(np.arange(n), np.diff(ia))
+    return ia, ja, a * (1.0 + 0.125 * (rows * sets // n))
+
+
+LOOSE = {  # lists that no row has all of, and lists padded to the next width
+    "six-sets": lambda n: _sets(n, (-97, -1, 0, 1, 97), 6),
+    "two-sets": lambda n: _sets(n, (-97, -1, 0, 1, 97), 2),
+    "tridiagonal": lambda n: _sets(n, (-1, 0, 1), 1),
+    "thirteen": lambda n: _sets(n, range(-6, 7), 1),
+    "box-27": lambda n: stencil_csr(n, box27(20, 400)),
+}
+
+
+@pytest.mark.parametrize("kind", sorted(LOOSE))
+def test_loose_stencils_take_any_kernel_alike(gpu_lib, kind):
+    """Operators whose stencil is timed among the other kernels: the filters and
+    products of the default route equal the SELL kernels' and the oracle's, and
+    KPM agrees with the general kernel's (the tolerance of test_kpm_on_stencils)."""
+    n = 12001
+    m = LOOSE[kind](n)
+    gpu_lib.set_csr(*m)
+    bound = float(np.abs(m[2]).max()) * 30
+    X = O.seeded_normal(5 * n, 9).reshape(5, n)
+    pols = [polynomial(gpu_lib, deg, bound)[0] for deg in (7, 4, 9, 2, 6)]
+    iv = [-0.2 * bound, 0.4 * bound, -bound, bound]
+    dX = E.DeviceBuffer.from_host(gpu_lib.lib, X)
+    try:
+        assert np.array_equal(gpu_lib.chebav(pols[0], X[0]), O.cheb_av(pols[0].as_dict(), *m, X[0]))
+        assert np.array_equal(gpu_lib.matvec(X[0]), O.csr_matvec(*m, X[0]))
+        assert np.array_equal(gpu_lib.matvec_cols(X)[4], O.csr_matvec(*m, X[4]))
+        for prec in (E.PREC_FP64, E.PREC_MIXED):
+            Y = gpu_lib.chebav_multi(pols, X, prec)
+            gpu_lib.set_filter_variant(0)
+            assert np.array_equal(Y, gpu_lib.chebav_multi(pols, X, prec)), prec
+            gpu_lib.set_filter_variant(-1)
+        dots = gpu_lib.kpm_dots(20, iv, dX, 5)
+        gpu_lib.set_row_patterns(False)
+        gpu_lib.set_csr(*m)
+        assert np.max(np.abs(dots - gpu_lib.kpm_dots(20, iv, dX, 5))) <= 4 * n * np.finfo(float).eps
+    finally:
+        gpu_lib.set_filter_variant(-1)
+        gpu_lib.set_row_patterns(True)
+
+
+@pytest.mark.parametrize("columns", [1, 16])
+def test_wide_lists_of_short_rows_do_not_take_the_stencil(gpu_lib, columns):
+    """Six sets of coefficients make a list of 30 entries for rows of 5: the
+    route taken is not the stencil, which costs about twice (16 columns) and
+    three times (one) what the dictionary's kernel does."""
+    import time
+
+    n = 600000
+    gpu_lib.set_csr(*_sets(n, (-775, -1, 0, 1, 775), 6))
+    lib = gpu_lib.lib
+    pol, mu = polynomial(gpu_lib, 40, 100.0)
+    pols = (E.PolParams * columns)(*[pol] * columns)
+    x, y = (E.DeviceBuffer.from_host(lib, np.zeros(n * columns)) for _ in range(2))
+    w = E.DeviceBuffer(lib, 24 * n)
+
+    def seconds(force):
+        gpu_lib.set_filter_kernel("merged-stencil" if force else None)
+        gpu_lib.set_filter_variant(8 if force else -1)
+        best = np.inf
+        for _ in range(4):
+            t = time.perf_counter()
+            if columns == 1:
+                assert lib.ChebAv(C.byref(pol), x.ptr, y.ptr, w.ptr) == 0
+            else:
+                assert lib.evslx_chebav_multi(columns, pols, x.ptr, y.ptr, E.PREC_FP64) == 0
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    try:
+        assert seconds(False) < 0.8 * seconds(True)
+        gpu_lib.set_filter_kernel(None)
+        assert columns > 1 or not gpu_lib.filter_stencil()
+    finally:
+        gpu_lib.set_filter_kernel(None)
+        gpu_lib.set_filter_variant(-1)
