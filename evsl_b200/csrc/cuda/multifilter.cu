@@ -903,7 +903,7 @@ int autotune(evslcu_mat *A, int fp32, int B) {
   evslcu_free(buf);
   // columns on a merged stencil that is not taken untimed
   float st_us = 0.0f;
-  if (!rc && stencil_ok(A) && !stencil_plain(A)) rc = stencil_columns_time(A, fp32, B, &st_us);
+  if (!rc && stencil_ok(A) && !stencil_plain(A) && (!fp32 || A->st_f32)) rc = stencil_columns_time(A, fp32, B, &st_us);
   if (!rc) {
     slot = (signed char)bestv;
     A->mf_cost_us[fp32 ? 1 : 0][log2_width(B)] = 1000.0f * best / steps;

@@ -98,6 +98,7 @@ struct evslcu_mat {
   int st_d = 0;
   int st_reach = 0;  // largest |offset|
   int st_span = 0;   // largest offset: rows r and r + st_span share most of what they gather
+  int st_f32 = 0;    // 1: every value is finite in FP32
   int st_plain = 0;  // 1: 5, 7 or 9 entries and a row that has them all
   void *st_mask = nullptr;
   double st_val[32] = {};

@@ -1594,11 +1594,12 @@ int stencil_build(evslcu_mat *M) {
       if ((int)list.size() > kStMax) return 0;
     }
   if (list.empty()) return 0;
-  int d = 0, reach = 0, span = 0;
+  int d = 0, reach = 0, span = 0, f32 = 1;
   for (auto &e : list) {
     e.second = d;
     M->st_off[d] = e.first.off;
     memcpy(&M->st_val[d], &e.first.bits, sizeof(double));
+    if (!std::isfinite((float)M->st_val[d])) f32 = 0;
     reach = std::max(reach, std::abs(e.first.off));
     span = std::max(span, e.first.off);
     ++d;
@@ -1629,6 +1630,7 @@ int stencil_build(evslcu_mat *M) {
   M->st_mask = dm;
   M->st_reach = reach;
   M->st_span = span;
+  M->st_f32 = f32;
   M->st_plain = (d == 5 || d == 7 || d == 9) && M->pat_maxlen == d;
   M->st_d = d;
   return 0;
@@ -1640,15 +1642,15 @@ void stencil_free(evslcu_mat *M) {
   M->st_d = M->st_plain = 0;
 }
 
-// Y(:, c) = A X(:, c) for m columns (1 <= m <= 65535).
+// Y(:, c) = A X(:, c) for m columns (1 <= m <= 65535) of a matrix that
+// stencil_spmv_ok takes.
 int stencil_spmv(const evslcu_mat *A, const double *X, double *Y, int m) {
   const dim3 g(grid_for(A->n), m);
   switch (st_width(A->st_d)) {
     case 5: k_st_spmv<5><<<g, kThreads, 0, stream()>>>(st_arg<double, 5>(A), X, Y, A->n); break;
     case 7: k_st_spmv<7><<<g, kThreads, 0, stream()>>>(st_arg<double, 7>(A), X, Y, A->n); break;
     case 9: k_st_spmv<9><<<g, kThreads, 0, stream()>>>(st_arg<double, 9>(A), X, Y, A->n); break;
-    case 16: k_st_spmv<16><<<g, kThreads, 0, stream()>>>(st_arg<double, 16>(A), X, Y, A->n); break;
-    default: k_st_spmv<32><<<g, kThreads, 0, stream()>>>(st_arg<double, 32>(A), X, Y, A->n); break;
+    default: k_st_spmv<16><<<g, kThreads, 0, stream()>>>(st_arg<double, 16>(A), X, Y, A->n); break;
   }
   EVSLCU_LAUNCH_CHECK("k_st_spmv");
   return 0;
@@ -1813,9 +1815,11 @@ static bool columns_apart(int n, int fp32, int ncols, const evslcu_filter_col *c
 }
 
 // Whether filter_columns takes these columns: a merged stencil, every degree
-// at least 1, and (once the vectors are known) no y in another column's way.
+// at least 1, values finite in the columns' precision (0 * inf would reach rows
+// without the entry), and (once the vectors are known) no y in another column's
+// way.
 bool stencil_columns_ok(const evslcu_mat *A, int fp32, int ncols, const evslcu_filter_col *cols, bool vectors) {
-  if (!stencil_ok(A)) return false;
+  if (!stencil_ok(A) || (fp32 && !A->st_f32)) return false;
   for (int c = 0; c < ncols; ++c)
     if (cols[c].deg < 1) return false;
   return !vectors || columns_apart(A->n, fp32, ncols, cols);

@@ -378,7 +378,8 @@ def test_loose_stencils_take_any_kernel_alike(gpu_lib, kind):
     gpu_lib.set_csr(*m)
     bound = float(np.abs(m[2]).max()) * 30
     X = O.seeded_normal(5 * n, 9).reshape(5, n)
-    pols = [polynomial(gpu_lib, deg, bound)[0] for deg in (7, 4, 9, 2, 6)]
+    made = [polynomial(gpu_lib, deg, bound) for deg in (7, 4, 9, 2, 6)]
+    pols = [p for p, _ in made]
     iv = [-0.2 * bound, 0.4 * bound, -bound, bound]
     dX = E.DeviceBuffer.from_host(gpu_lib.lib, X)
     try:
@@ -397,6 +398,28 @@ def test_loose_stencils_take_any_kernel_alike(gpu_lib, kind):
     finally:
         gpu_lib.set_filter_variant(-1)
         gpu_lib.set_row_patterns(True)
+
+
+def test_values_beyond_fp32_stay_in_their_rows(gpu_lib):
+    """A value that is infinite in FP32, in the last rows only: FP32 columns are
+    infinite or not a number where the general kernel's are, and equal elsewhere
+    (an absent entry must not become 0 * inf)."""
+    n = 2000
+    ia, ja, a = stencil_csr(n, SHAPES["cluster-exact"][1])
+    a = a.copy()
+    a[ia[1900]:] *= 1e39
+    gpu_lib.set_csr(ia, ja, a)
+    made = [polynomial(gpu_lib, deg, 8.0) for deg in (3, 5)]
+    pols = [p for p, _ in made]
+    X = O.seeded_normal(2 * n, 4).reshape(2, n)
+    try:
+        Y = gpu_lib.chebav_multi(pols, X, E.PREC_MIXED)
+        gpu_lib.set_filter_variant(0)
+        ref = gpu_lib.chebav_multi(pols, X, E.PREC_MIXED)
+    finally:
+        gpu_lib.set_filter_variant(-1)
+    assert np.array_equal(Y, ref, equal_nan=True)
+    assert np.all(np.isfinite(Y[:, :1400])) and not np.any(np.isfinite(Y[:, 1900:]))
 
 
 @pytest.mark.parametrize("columns", [1, 16])
