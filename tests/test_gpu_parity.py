@@ -642,14 +642,26 @@ def test_filter_kernels_on_nine_entry_rows(gpu_lib, variant):
 
 
 @pytest.mark.parametrize("nvec", [20, 13])
-def test_kpm_prefetch_form_is_bitwise(gpu_lib, nvec):
+@pytest.mark.parametrize("matrix", ["rspd", "wide-dictionary"])
+def test_kpm_prefetch_form_is_bitwise(gpu_lib, matrix, nvec):
     """The KPM block step that loads each row's own v_k, v_k-1 before its
     gathers (and stores 16 bytes at a time) performs the same operations:
     its raw dot products equal the default form's bit for bit, even and odd
-    probe counts (paired and single loads)."""
+    probe counts (paired and single loads), on stored entries and on a
+    row-pattern dictionary (one without a merged stencil, which has a KPM of
+    its own)."""
     import evsl_b200
+    from evsl_b200 import workloads as W
 
-    ia, ja, a = _lap(gpu_lib, 14, 12, 5)
+    if matrix == "rspd":
+        ia, ja, a = W.random_spd_csr(1200, 8, 3)
+    else:
+        n = 1500  # 41 offsets: the dictionary's patterns do not merge into 32 entries
+        ia, ja, a = _csr_from_rows([([c for c in range(r - 20, r + 21) if 0 <= c < n],
+                                     [5.5 if c == r else -0.1 for c in range(r - 20, r + 21) if 0 <= c < n])
+                                    for r in range(n)])
+    gpu_lib.set_csr(ia, ja, a)
+    assert (gpu_lib.row_pattern_count() > 0) == (matrix == "wide-dictionary") and not gpu_lib.filter_stencil()
     n = len(ia) - 1
     iv = [0.7, 2.9, 0.0, 12.0]
     probes = evsl_b200.DeviceBuffer.from_host(gpu_lib.lib, O.seeded_rademacher(nvec, n, 5))

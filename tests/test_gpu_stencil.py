@@ -114,19 +114,46 @@ def test_stencil_filter_is_bitwise(gpu_lib, shape, blocks):
 
 
 def test_dictionaries_that_do_not_merge_keep_the_other_kernels(gpu_lib):
-    """More than 32 entries, and rows whose columns do not increase."""
+    """More than 32 entries, and rows whose columns do not increase: the filter,
+    the products, several columns (against the SELL kernel) and KPM (against the
+    matrix without its dictionary, with the tolerance of test_kpm_on_stencils,
+    and bitwise with the prefetching form)."""
     wide = stencil_csr(2000, [(o, 1.0 / (50 + o)) for o in range(-20, 21)])
     ia, ja, a = stencil_csr(2000, [(-30, -1.0), (-1, -1.0), (0, 4.0), (1, -1.0), (30, -1.0)])
     ja, a = ja.copy(), a.copy()
     for r in range(0, 2000, 2):
         ja[ia[r]:ia[r + 1]] = ja[ia[r]:ia[r + 1]][::-1]
         a[ia[r]:ia[r + 1]] = a[ia[r]:ia[r + 1]][::-1]
-    for m in (wide, (ia, ja, a)):
-        gpu_lib.set_csr(*m)
-        assert gpu_lib.row_pattern_count() > 0
-        v = O.seeded_normal(2000, 3)
-        pol, mu = polynomial(gpu_lib, 7, 8.0)
-        assert np.array_equal(gpu_lib.chebav(pol, v), O.cheb_av(pol.as_dict(), *m, v))
+    iv = [0.4, 2.9, -8.0, 8.0]
+    X = O.seeded_normal(3 * 2000, 3).reshape(3, 2000)
+    dX = E.DeviceBuffer.from_host(gpu_lib.lib, X)
+    pol, mu = polynomial(gpu_lib, 7, 8.0)
+    try:
+        for m in (wide, (ia, ja, a)):
+            gpu_lib.set_csr(*m)
+            assert gpu_lib.row_pattern_count() > 0 and not gpu_lib.filter_stencil()
+            assert np.array_equal(gpu_lib.chebav(pol, X[0]), O.cheb_av(pol.as_dict(), *m, X[0]))
+            Y = gpu_lib.matvec_cols(X)
+            for c in range(3):
+                assert np.array_equal(Y[c], O.csr_matvec(*m, X[c]))
+                assert np.array_equal(Y[c], gpu_lib.matvec(X[c]))
+            for prec in (E.PREC_FP64, E.PREC_MIXED):
+                Y = gpu_lib.chebav_multi([pol] * 3, X, prec)
+                gpu_lib.set_filter_variant(0)
+                assert np.array_equal(Y, gpu_lib.chebav_multi([pol] * 3, X, prec)), prec
+                gpu_lib.set_filter_variant(-1)
+            dots = gpu_lib.kpm_dots(21, iv, dX, 3)
+            gpu_lib.lib.evslcu_set_kpm_prefetch(1)
+            assert np.array_equal(dots, gpu_lib.kpm_dots(21, iv, dX, 3))
+            gpu_lib.lib.evslcu_set_kpm_prefetch(0)
+            gpu_lib.set_row_patterns(False)
+            gpu_lib.set_csr(*m)
+            assert np.max(np.abs(dots - gpu_lib.kpm_dots(21, iv, dX, 3))) <= 4 * 2000 * np.finfo(float).eps
+            gpu_lib.set_row_patterns(True)
+    finally:
+        gpu_lib.set_filter_variant(-1)
+        gpu_lib.lib.evslcu_set_kpm_prefetch(0)
+        gpu_lib.set_row_patterns(True)
 
 
 MULTI = ["cluster-over", "dropped-7", "eleven", "box-9", "lopsided", "two-rows-5", "two-rows-dropped",
