@@ -1176,6 +1176,7 @@ int cl_chebav(const evslcu_mat *A, const double *mu, int deg, double cc, double 
               const evslcu_cheb_epi *epi, bool *done) {
   if (A->st_d > kClMaxD || g_cl_force < 0) return 0;
   const int most = deg < 64 ? cl_most<double, 64>(A->st_d) : deg < 512 ? cl_most<double, 512>(A->st_d) : cl_most<double, 0>(A->st_d);
+  if (most < 1) return 0;
   // One cluster of all the blocks it may have; a block alone below kClOneBlock
   // rows, where a degree costs less than the exchange of halos.  Measured on
   // 16 blocks, us a degree: 0.48 on 1,480 rows, 0.52 on 10^4 (2-D), 0.60 on 6,840
