@@ -79,8 +79,8 @@ typedef struct req_s {
   struct req_s *next;
 } req_t;
 
-/* A captured filter (CUDA graph) for the slots of one matrix, valid while
- * the same requests occupy them in the same order. */
+/* A prepared filter (evslcu_filter_plan) for the slots of one matrix, valid
+ * while the same requests occupy them in the same order. */
 typedef struct {
   evslx_matrix *M;
   int ncols, used;
@@ -355,8 +355,8 @@ void evslx_engine_group_widths(const evslx_engine *E, uint64_t counts[5]) {
 }
 
 /* Runs the filters of the nc columns cols (all on M, request ids uids)
- * through a cached graph when the same requests were filtered together
- * before, else captures one (or, with graphs off, launches directly). */
+ * through a cached plan when the same requests were filtered together before,
+ * else makes one (or, with plans off, launches directly). */
 static int run_group_filter(evslx_engine *E, evslx_matrix *M, int nc, const evslcu_filter_col *cols,
                             const uint64_t *uids, int fp32) {
   int wb = 0;

@@ -321,8 +321,11 @@ int evslx_engine_step(evslx_engine *E);
  * matrices with at least `rows` rows (default 131072) and filter smaller ones
  * in FP64, where FP32 saves little and the refinement costs more. */
 void evslx_set_mixed_min_rows(int rows);
-/* Filters run as captured CUDA graphs, rebuilt when the set of requests on
- * a matrix changes (default on); plan_builds counts the captures. */
+/* Filters of several columns run from plans, rebuilt when the set of requests
+ * on a matrix changes (default on; off: each call prepares its own): a captured
+ * CUDA graph, or, where the columns run on the matrix's merged stencil, their
+ * coefficients on the device and direct launches, of which there are few.
+ * plan_builds counts the plans of either kind. */
 void evslx_engine_use_graphs(evslx_engine *E, int on);
 /* Batched filter of the engine (default on, max_rows 2^18): every tick, the
  * lone FP64 columns of matrices with at most max_rows rows (independent
