@@ -1255,7 +1255,7 @@ int cheb_variant(const evslcu_mat *A_) {
   if (A->kernel != 0) return -1;
   // a matrix with a plain merged stencil claims constant memory only when the
   // variants that read it are asked for
-  if (A->st_plain && A->pat_chdr < 0 && pat_const_claim(A)) return EVSLCU_ERR_CUDA;
+  if (A->st_plain && g_cheb_force != kChebStencil && A->pat_chdr < 0 && pat_const_claim(A)) return EVSLCU_ERR_CUDA;
   if (g_cheb_force == 7 && panel_candidate(A) && !A->pn64) {
     const int prc = panel_build(A, 0);
     if (prc) return prc;

@@ -217,6 +217,58 @@ def test_engine_batch_of_stencils_of_all_widths(gpu_lib):
         gpu_lib.free_pol(p)
 
 
+@pytest.mark.parametrize("shape", ["cluster-over", "cluster-halo-rows", "cluster-loop"])
+def test_long_filters_on_a_cluster_are_bitwise(gpu_lib, shape):
+    """Degrees around the sizes at which a cluster filter's coefficients change
+    place (63 and 511 in the launch's arguments, more on the device), with every
+    remainder of the loop over three degrees."""
+    n, entries, drop = SHAPES[shape]
+    ia, ja, a = stencil_csr(n, entries, drop)
+    gpu_lib.set_csr(ia, ja, a)
+    v = O.seeded_normal(n, 3)
+    try:
+        for deg in (10, 35, 63, 64, 65, 511, 512, 700):
+            pol, mu = polynomial(gpu_lib, deg, 1.2 * sum(abs(v) for _, v in entries))
+            gpu_lib.set_filter_kernel("merged-stencil")
+            before = gpu_lib.launch_count()
+            y = gpu_lib.chebav(pol, v)
+            assert gpu_lib.launch_count() - before == 1
+            gpu_lib.set_filter_kernel(0)
+            assert np.array_equal(y, gpu_lib.chebav(pol, v)), deg
+    finally:
+        gpu_lib.set_filter_kernel(-1)
+
+
+def test_engine_batch_with_halos_of_most_of_a_block(gpu_lib):
+    """Operators whose largest offset is a third to a half of their rows, beside
+    one with short offsets, filtered together on clusters: the same eigenvalues
+    as with each matrix's own filter."""
+    five = lambda s: [(-s, -1.0), (-1, -1.0), (0, 4.2), (1, -1.0), (s, -1.0)]  # noqa: E731
+    ops = [(700, five(230)), (1003, five(480)), (1600, five(40)), (2048, five(1000))]
+    mats = [gpu_lib.matrix(*stencil_csr(n, e)) for n, e in ops]
+    iv = [3.0, 3.1, 0.0, 8.4]
+    pol = gpu_lib.find_pol(iv, max_deg=300)
+    out = []
+    for batch in (True, False):
+        eng = gpu_lib.engine(len(ops), precision=E.PREC_FP64)
+        eng.use_batch(batch)
+        for t, (n, _) in enumerate(ops):
+            eng.submit_slice(mats[t], iv, pol, 200, 1e-8, O.seeded_normal(n, t), t)
+        eng.run()
+        got = {}
+        while (r := eng.pop()) is not None:
+            got[r["tag"]] = r["lam"]
+        assert (eng.batched_columns() > 0) == batch
+        eng.free()
+        out.append(got)
+    assert len(out[0]) == len(ops) and sum(len(lam) for lam in out[0].values()) > 0
+    for t in out[0]:
+        assert np.array_equal(out[0][t], out[1][t]), t
+    for m in mats:
+        m.free()
+    gpu_lib.free_pol(pol)
+
+
 @pytest.mark.parametrize("blocks", [-1, 0, 1])
 @pytest.mark.parametrize("shape", ["one-row", "tridiagonal", "cluster-over", "cluster-loop", "dropped-7", "eleven",
                                    "box-9", "two-rows-7"])
