@@ -13,8 +13,8 @@
 //     term), and adding them one after another is the same sum in the same
 //     order at 16 / 3 instead of 16 bytes of y per row and degree.
 //     Against the dictionary kernels before it (sparse.cu, the fastest of the
-//     seven timed): 3-D Laplacian of 10^6 rows 7.84 -> 6.49 us a degree, 343
-//     thousand rows 4.57 -> 3.56, 10^4 rows 2.95 -> 2.4 (launch latency).
+//     seven timed): 3-D Laplacian of 10^6 rows 7.84 -> 6.32 us a degree, 343
+//     thousand rows 4.57 -> 3.18, 10^4 rows 2.95 -> 2.4 (launch latency).
 //   * k_st_cluster: every degree in one launch, for operators whose vectors
 //     fit the shared memory of one thread-block cluster: 10^4 rows 2.4 -> 0.52.
 //   * k_st_cols, k_st_clusters: the same two for several columns, each with
@@ -48,6 +48,7 @@ __global__ void k_st_mask(int n, const unsigned short *__restrict__ pid, const u
 struct StMarch {
   int S, J, cols;
   unsigned magic;  // floor(2^32 / S)
+  int ahead;       // one column: blocks that run at once, and so beside the launch ahead
 };
 
 // What a degree does to y: terms pending since y was last written (0: none
@@ -64,12 +65,14 @@ struct StY {
 // Returns the sum of dotv[r] y[r] over the thread's rows (EPI).  yd: where the
 // finished y goes (the last degree), else null.
 // each(x, w) is called for every row, with its values of v_k and of the result.
-// OWN (J > 1): a row's own v_k is loaded before the masks are looked at.
-template <class VT, int D, int J, bool FIRST, bool EPI, bool OWN, class F>
+// LONE: one column's launch.  Its first blocks prefetch v_k-1, and with J > 1 a
+// row's own v_k is loaded before the masks are looked at.
+template <class VT, int D, int J, bool FIRST, bool EPI, bool LONE, class F>
 __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &M, const VT *__restrict__ vk,
                                           const VT *vkm1, VT *out, VT *y, double *yd, VT t, VT ncc, const StY<VT> &Y,
                                           const double *__restrict__ zold, double nbeta,
                                           const double *__restrict__ dotv, F &&each) {
+  constexpr bool OWN = LONE && J > 1;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   int r0 = c;
   if (J > 1) {
@@ -83,12 +86,14 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
   }
   // Only the masks are loaded before the wait: the host has waited for the
   // kernel that wrote them (stencil_build).  v_k-1 was written two launches
-  // ago, but it is the wait that makes other launches' writes visible.  (Loaded
-  // before it, v_k-1 overlapped the launch ahead: 3.15 instead of 3.56 us a
-  // degree on 343 thousand rows, 6.30 instead of 6.49 on 10^6.)  What needs no
-  // mask is loaded before the masks are looked at, which costs the blocks that
-  // start after the wait no second latency: 10^6 rows 6.87 -> 6.49; OWN gains in
-  // one column's launches and loses where many columns fill the chip.
+  // ago, but it is the wait that makes other launches' writes visible; before it
+  // the blocks that start beside the launch ahead may only ask for it to be
+  // brought near: 343 thousand rows 3.55 -> 3.18 us a degree, 10^6 6.50 -> 6.32
+  // (6.54 when the blocks of later waves ask as well).  What needs no mask is
+  // loaded before the masks are looked at, which costs the blocks that start
+  // after the wait no second latency: 10^6 rows 6.87 -> 6.50.  The prefetch and
+  // the early own row gain in one column's launches and lose where many columns
+  // fill the chip.
   unsigned m[J];
   bool live[J];
   bool all = true;
@@ -97,6 +102,8 @@ __device__ __forceinline__ double st_rows(const StArg<VT, D> &A, const StMarch &
     const int r = r0 + j * M.S;
     live[j] = r < A.n;
     m[j] = live[j] ? (unsigned)__ldg(A.mask + r) : 0u;
+    if (LONE && !FIRST && live[j] && (int)blockIdx.x < M.ahead)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(vkm1 + r));
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -213,8 +220,8 @@ __global__ void __launch_bounds__(kThreads, J == 2 ? 5 : D <= 9 ? 6 : 2)
               const double *__restrict__ zold, double nbeta, const double *__restrict__ dotv, double *part,
               unsigned int *ctr, double *dot_out) {
   __shared__ double sh[EPI ? kThreads / 32 : 1];
-  const double dsum = st_rows<double, D, J, FIRST, EPI, J == 2>(A, M, vk, vkm1, out, y, yd, t, ncc, Y, zold, nbeta,
-                                                                dotv, [](double, double) {});
+  const double dsum = st_rows<double, D, J, FIRST, EPI, true>(A, M, vk, vkm1, out, y, yd, t, ncc, Y, zold, nbeta, dotv,
+                                                              [](double, double) {});
   if (EPI && dot_out) {
     const double b = block_sum(dsum, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = b;
@@ -342,10 +349,11 @@ __global__ void k_st_float(int n, const double *__restrict__ x, float *out) {
 // Two rows per thread: FP64 columns and probes from kStTwoRows rows on; FP32
 // columns also, and one column only, where one row per thread would need more
 // blocks than run at once (6 on an SM).
-// Measured, us a degree of one column, 1 / 2 rows per thread: 215 thousand rows
-// 2.73 / 3.41, 343 thousand 3.57 / 3.56, 450 thousand 3.81 / 4.17, 592 thousand
-// 4.50 / 4.59, 10^6 (3-D) 6.35 / 6.49, 10^6 (2-D) 5.74 / 5.37, 4.1 million
-// 25.3 / 25.3; three rows were 4-8% slower than two at every size.  FP32 columns
+// Measured before v_k-1 was prefetched, us a degree of one column, 1 / 2 rows per
+// thread: 215 thousand rows 2.73 / 3.41, 343 thousand 3.57 / 3.56, 450 thousand
+// 3.81 / 4.17, 592 thousand 4.50 / 4.59, 10^6 (3-D) 6.35 / 6.49, 10^6 (2-D) 5.74 /
+// 5.37, 4.1 million 25.3 / 25.3; three rows were 4-8% slower than two at every
+// size.  FP32 columns
 // of a 5-point operator: 100 thousand rows x 16 9.82 / 7.43 (the packing kernel
 // 8.64), x 4 3.76 / 3.14, 40 thousand x 8 3.55 / 3.16; FP64, 9 points: 100
 // thousand x 16 10.5 / 10.7, x 4 4.08 / 4.84.
@@ -358,6 +366,7 @@ StMarch st_march(int n, int span, bool sym, bool two) {
   if (!sym || span < 1 || (long long)span * J > n || n > (1 << 29)) J = 1;
   M.S = J > 1 ? span : std::max(n, 1);
   M.J = J;
+  M.ahead = 0;
   const long long groups = ((long long)n + (long long)M.S * J - 1) / ((long long)M.S * J);
   M.cols = (int)(groups * M.S);
   M.magic = (unsigned)((1ull << 32) / (unsigned long long)M.S - (M.S == 1 ? 1 : 0));
@@ -368,7 +377,8 @@ template <int D>
 int st_step(const evslcu_mat *A, bool first, const double *vk, const double *vkm1, double *out, double *y, double t,
             double ncc, const StY<double> &Y, bool last, const evslcu_cheb_epi *ep) {
   const StArg<double, D> S = st_arg<double, D>(A);
-  const StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], st_over_one_wave(A->n));
+  StMarch M = st_march(A->n, A->st_span, D <= 9 && S.center && S.off[0] == -S.off[D - 1], st_over_one_wave(A->n));
+  M.ahead = sm_count() * (M.J == 2 ? 5 : 6);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M.cols + kThreads - 1) / kThreads);
   cfg.blockDim = dim3(kThreads);
