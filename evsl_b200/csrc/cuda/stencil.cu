@@ -534,9 +534,11 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
 }
 // The end of a block that gave up, after a cluster barrier that the others
 // reach (or leave the kernel) without sending again: values already on their
-// way to its shared memory need a microsecond or two to arrive.
+// way to its shared memory need a microsecond or two to arrive; this is about a
+// hundred.
 __device__ __forceinline__ void linger() {
-  for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  const long long t = clock64();
+  while (clock64() - t < 200000) __nanosleep(1000);
 }
 
 // Shared memory: two vectors of R rows with a halo on both sides, which take
